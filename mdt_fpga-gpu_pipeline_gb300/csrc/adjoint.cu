@@ -17,70 +17,196 @@
 
 namespace mdt {
 
-// Y[c][s][e] = g[c][e] * X[c][s][e] (complex gains on the F-engine output).
-__global__ void apply_gains_kernel(long n, int ne, int nsp, const float2 *__restrict__ X,
-                                   const float2 *__restrict__ g, float2 *__restrict__ Y)
+// Compensated dot products: hi + lo accumulates sum a*b with every rounding
+// error of the products and of the sum carried along in lo (Dot2 of Ogita,
+// Rump and Oishi, "Accurate sum and dot product", SIAM J. Sci. Comput. 26,
+// 2005), which is as accurate as a sum in twice the working precision (2^-48).
+// The GPU's FP64 rate is a hundredth of its FP32 rate: sums kept in double
+// held the two gradient kernels below on the FP64 pipe.  Infinities and NaN
+// leave NaN in lo; the kernels then repeat the thread's sum in double.
+struct Sum2 {
+    float hi = 0.0f, lo = 0.0f;
+    __device__ __forceinline__ void add(float a, float b)
+    {
+        const float p = __fmul_rn(a, b);
+        const float e = __fmaf_rn(a, b, -p);
+        const float s = __fadd_rn(hi, p);
+        const float v = __fsub_rn(s, hi);
+        const float d = __fadd_rn(__fsub_rn(hi, __fsub_rn(s, v)), __fsub_rn(p, v));
+        hi = s;
+        lo = __fadd_rn(lo, __fadd_rn(e, d));
+    }
+    __device__ __forceinline__ bool finite() const { return isfinite(hi) && isfinite(lo); }
+    __device__ __forceinline__ double value() const { return (double)hi + (double)lo; }
+};
+struct SumD {
+    double v = 0.0;
+    __device__ __forceinline__ void add(float a, float b) { v += (double)a * (double)b; }
+    __device__ __forceinline__ bool finite() const { return true; }
+    __device__ __forceinline__ double value() const { return v; }
+};
+
+// VEC consecutive complex64 values (VEC 2: 16-byte aligned).
+template <int VEC>
+__device__ __forceinline__ void load_c64(const float2 *p, float2 (&v)[VEC])
 {
-    const long j = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    const long e = j % ne, c = j / ((long)nsp * ne);
-    Y[j] = cmul(g[c * ne + e], X[j]);
+    if constexpr (VEC == 2) {
+        const float4 t = __ldg(reinterpret_cast<const float4 *>(p));
+        v[0] = make_float2(t.x, t.y);
+        v[1] = make_float2(t.z, t.w);
+    } else {
+        v[0] = __ldg(p);
+    }
 }
 
-// dg[c][e] = sum_s dY[c][s][e] * conj(X[c][s][e]).  32 (c, e) pairs per block,
-// 8 spectrum phases per pair summed in double and combined in a fixed order.
-__global__ void gain_grad_kernel(int ne, int nch, int nsp, const float2 *__restrict__ dY,
-                                 const float2 *__restrict__ X, float2 *__restrict__ dg)
+// Y[c][s][e] = g[c][e] * X[c][s][e] (complex gains on the F-engine output).
+// Bound by HBM (16 bytes a value).  A block covers AG_ITEMS vectors of VEC
+// elements per thread, a block's width apart, so that the element index is
+// one division per thread and then steps without one, and every access is 16
+// bytes wide (VEC 2: NE even and 16-byte buffers; otherwise one value).
+// NE=64, Nch=512, Nsp=2048: 157 us (6.8 TB/s); one value and two 64-bit
+// divisions per thread took 277 us.
+constexpr int AG_THREADS = 256, AG_ITEMS = 4;
+template <int VEC>
+__global__ void __launch_bounds__(AG_THREADS)
+    apply_gains_kernel(int nch, int ne, long per, int step, const float2 *__restrict__ X,
+                       const float2 *__restrict__ g, float2 *__restrict__ Y)
 {
-    __shared__ double sre[8][33], sim[8][33];
-    const long j = (long)blockIdx.x * 32 + threadIdx.x;
-    const int ph = threadIdx.y;
-    double re = 0.0, im = 0.0;
-    if (j < (long)nch * ne) {
-        const long c = j / ne, e = j - c * ne;
-        const long base = c * nsp * (long)ne + e;
-        for (int s = ph; s < nsp; s += 8) {
-            const float2 a = dY[base + (long)s * ne], b = X[base + (long)s * ne];
-            re += (double)a.x * b.x + (double)a.y * b.y;
-            im += (double)a.y * b.x - (double)a.x * b.y;
+    // per = Nsp * NE / VEC vectors of a channel; step = AG_THREADS * VEC mod NE
+    const long i0 = (long)blockIdx.x * (AG_THREADS * AG_ITEMS) + threadIdx.x;
+    if (i0 >= per) return;
+    const int e0 = (int)((i0 * VEC) % ne);
+    for (int c = blockIdx.y; c < nch; c += gridDim.y) {
+        const float2 *xc = X + (long)c * per * VEC, *gc = g + (long)c * ne;
+        float2 *yc = Y + (long)c * per * VEC;
+        int e = e0;
+#pragma unroll
+        for (int k = 0; k < AG_ITEMS; k++) {
+            const long i = i0 + k * AG_THREADS;
+            if (i < per) {
+                float2 x[VEC], gv[VEC];
+                load_c64<VEC>(xc + i * VEC, x);
+                load_c64<VEC>(gc + e, gv);
+                if constexpr (VEC == 2) {
+                    const float2 a = cmul(gv[0], x[0]), b = cmul(gv[1], x[1]);
+                    *reinterpret_cast<float4 *>(yc + i * 2) = make_float4(a.x, a.y, b.x, b.y);
+                } else {
+                    yc[i] = cmul(gv[0], x[0]);
+                }
+            }
+            e += step;
+            if (e >= ne) e -= ne;
         }
     }
-    sre[ph][threadIdx.x] = re;
-    sim[ph][threadIdx.x] = im;
-    __syncthreads();
-    if (ph == 0 && j < (long)nch * ne) {
-        for (int p = 1; p < 8; p++) {
-            re += sre[p][threadIdx.x];
-            im += sim[p][threadIdx.x];
+}
+
+// dg[c][e] = sum_s dY[c][s][e] * conj(X[c][s][e]).  32 vectors of VEC (c, e)
+// pairs per block, GG_PH spectrum phases per pair (compensated FP32 sums),
+// combined in double in a fixed order.  Bound by HBM (16 bytes a value); four
+// blocks of eight warps per SM keep enough 16-byte loads in flight (two blocks
+// of sixteen: 320 us).  NE=64, Nch=512, Nsp=2048: 172 us (6.2 TB/s); sums in
+// double took 1284 us.
+constexpr int GG_PH = 8;
+template <int VEC, class Sum>
+__device__ __forceinline__ bool gain_sums(int ne, int nsp, int ph, const float2 *dY,
+                                          const float2 *X, double (&re)[VEC], double (&im)[VEC])
+{
+    Sum ar[VEC], ai[VEC];
+#pragma unroll 4
+    for (int s = ph; s < nsp; s += GG_PH) {
+        float2 a[VEC], b[VEC];
+        load_c64<VEC>(dY + (long)s * ne, a);
+        load_c64<VEC>(X + (long)s * ne, b);
+#pragma unroll
+        for (int v = 0; v < VEC; v++) {
+            ar[v].add(a[v].x, b[v].x);
+            ar[v].add(a[v].y, b[v].y);
+            ai[v].add(a[v].y, b[v].x);
+            ai[v].add(-a[v].x, b[v].y);
         }
-        dg[j] = make_float2((float)re, (float)im);
+    }
+    bool ok = true;
+#pragma unroll
+    for (int v = 0; v < VEC; v++) {
+        ok = ok && ar[v].finite() && ai[v].finite();
+        re[v] = ar[v].value();
+        im[v] = ai[v].value();
+    }
+    return ok;
+}
+
+template <int VEC>
+__global__ void __launch_bounds__(32 * GG_PH, 4)
+    gain_grad_kernel(int ne, int nch, int nsp, const float2 *__restrict__ dY,
+                     const float2 *__restrict__ X, float2 *__restrict__ dg)
+{
+    __shared__ double sre[GG_PH][32 * VEC + 1], sim[GG_PH][32 * VEC + 1];
+    const int ev = ne / VEC;
+    const long j = (long)blockIdx.x * 32 + threadIdx.x;
+    const int ph = threadIdx.y;
+    const bool in = j < (long)nch * ev;
+    double re[VEC] = {}, im[VEC] = {};
+    if (in) {
+        const long c = j / ev, e = (j - c * ev) * VEC;
+        const long base = c * nsp * (long)ne + e;
+        if (!gain_sums<VEC, Sum2>(ne, nsp, ph, dY + base, X + base, re, im))
+            gain_sums<VEC, SumD>(ne, nsp, ph, dY + base, X + base, re, im);
+    }
+#pragma unroll
+    for (int v = 0; v < VEC; v++) {
+        sre[ph][threadIdx.x * VEC + v] = re[v];
+        sim[ph][threadIdx.x * VEC + v] = im[v];
+    }
+    __syncthreads();
+    if (ph == 0 && in) {
+#pragma unroll
+        for (int v = 0; v < VEC; v++) {
+            for (int p = 1; p < GG_PH; p++) {
+                re[v] += sre[p][threadIdx.x * VEC + v];
+                im[v] += sim[p][threadIdx.x * VEC + v];
+            }
+            dg[j * VEC + v] = make_float2((float)re[v], (float)im[v]);
+        }
     }
 }
 
 // Adjoint of the gains and of the channel-major reorder:
-// dF[s][e][c] = conj(g[c][e]) * dY[c][s][e] -- a 32 x 32 tiled transpose of
-// (channel) x (spectrum, element) rows.
-__global__ void fout_adjoint_kernel(int ne, int nch, long rows, const float2 *__restrict__ dY,
-                                    const float2 *__restrict__ g, float2 *__restrict__ dF)
+// dF[s][e][c] = conj(g[c][e]) * dY[c][s][e] -- a FA_T x FA_T tiled transpose
+// of (channel) x (spectrum, element) rows.  Bound by HBM (16 bytes a value):
+// eight independent loads per thread, the element index formed once per
+// thread and row half.  NE=64, Nch=512, Nsp=2048: 210 us (5.1 TB/s), with
+// 32 x 32 tiles and a 64-bit division per value 233 us.
+constexpr int FA_T = 64;
+__global__ void __launch_bounds__(512)
+    fout_adjoint_kernel(int ne, int nch, long rows, const float2 *__restrict__ dY,
+                        const float2 *__restrict__ g, float2 *__restrict__ dF)
 {
-    __shared__ float2 t[32][33];
-    const long r0 = (long)blockIdx.x * 32;
-    const int c0 = blockIdx.y * 32;
-    for (int y = threadIdx.y; y < 32; y += 8) {
-        const int c = c0 + y;
-        const long r = r0 + threadIdx.x;
-        float2 v = make_float2(0.f, 0.f);
-        if (c < nch && r < rows) {
-            const float2 gv = g ? g[(long)c * ne + r % ne] : make_float2(1.f, 0.f);
-            v = cmul(cconj(gv), dY[(long)c * rows + r]);
+    __shared__ float2 t[FA_T][FA_T + 1];
+    const long r0 = (long)blockIdx.x * FA_T;
+    const int c0 = blockIdx.y * FA_T, lane = threadIdx.x, warp = threadIdx.y;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const long r = r0 + 32 * h + lane;
+        const int e = (int)(r % ne);
+#pragma unroll
+        for (int y = 0; y < FA_T / 16; y++) {
+            const int c = c0 + warp + 16 * y;
+            if (c < nch && r < rows) {
+                const float2 gv = g ? __ldg(g + (long)c * ne + e) : make_float2(1.f, 0.f);
+                t[warp + 16 * y][32 * h + lane] = cmul(cconj(gv), __ldg(dY + (long)c * rows + r));
+            }
         }
-        t[y][threadIdx.x] = v;
     }
     __syncthreads();
-    for (int y = threadIdx.y; y < 32; y += 8) {
-        const long r = r0 + y;
-        const int c = c0 + threadIdx.x;
-        if (c < nch && r < rows) dF[r * nch + c] = t[threadIdx.x][y];
+#pragma unroll
+    for (int y = 0; y < FA_T / 16; y++) {
+        const long r = r0 + warp + 16 * y;
+        if (r >= rows) continue;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const int c = c0 + 32 * h + lane;
+            if (c < nch) dF[r * nch + c] = t[32 * h + lane][warp + 16 * y];
+        }
     }
 }
 
@@ -149,43 +275,124 @@ __global__ void pfb_tap_grad_partial_kernel(int nch, int ntaps, int ne, int nsp,
     part[((long)p * ntaps + i) * nch + k] = acc;
 }
 
-// All taps at once (Ntaps <= 16): gP is read once, the int8 input of the
-// NT taps from L2.  part[p][i][k] as above.
-template <int NT>
-__global__ void pfb_tap_grad_all_kernel(int nch, int ne, int nsp, int nsplit,
-                                        const float2 *__restrict__ gP,
-                                        const char2 *__restrict__ iq, double *__restrict__ part)
+// NT = 4 or 8 taps at once: part[p][i][k] as above.  A thread owns VEC
+// channels and walks runs of TG_RUN spectra of one element, so that every
+// gradient value and (but for the NT-1 spectra of a run's lead-in) every
+// sample is read once; the samples of the NT taps rotate through registers.
+// The runs are dealt to the TG_PH warps of a block and to the splits in turn;
+// each thread's sums are compensated FP32, combined in double in a fixed
+// order.  Bound by the FP32 pipe (10 operations a product; 145 us at NE=64,
+// Nch=512, 4 taps, Nsp=2048) and by latency: 265 us there, 3328 us with sums
+// in double.
+constexpr int TG_PH = 16, TG_RUN = 32;
+
+template <int VEC>
+__device__ __forceinline__ void load_iq(const char2 *p, float (&re)[VEC], float (&im)[VEC])
 {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    const int p = blockIdx.y;
-    if (k >= nch) return;
-    const long rows = (long)nsp * ne;
-    const long r0 = rows * p / nsplit, r1 = rows * (p + 1) / nsplit;
-    double acc[NT];
-#pragma unroll
-    for (int i = 0; i < NT; i++) acc[i] = 0.0;
-    for (long row = r0; row < r1; row++) {
-        const long s = row / ne, e = row - s * ne;
-        const float2 g = gP[row * nch + k];
-#pragma unroll
-        for (int i = 0; i < NT; i++) {
-            const char2 x = iq[((s + i) * ne + e) * nch + k];
-            acc[i] += (double)g.x * (double)x.x + (double)g.y * (double)x.y;
-        }
+    if constexpr (VEC == 2) {
+        const char4 t = __ldg(reinterpret_cast<const char4 *>(p));
+        re[0] = (float)t.x;
+        im[0] = (float)t.y;
+        re[1] = (float)t.z;
+        im[1] = (float)t.w;
+    } else {
+        const char2 t = __ldg(p);
+        re[0] = (float)t.x;
+        im[0] = (float)t.y;
     }
-#pragma unroll
-    for (int i = 0; i < NT; i++) part[((long)p * NT + i) * nch + k] = acc[i];
 }
 
-// gW[i][k] = sum_p part[p][i][k] in increasing p (deterministic).
-__global__ void pfb_tap_grad_reduce_kernel(int n, int nsplit, const double *__restrict__ part,
-                                           float *__restrict__ gW)
+template <int NT, int VEC, class Sum>
+__device__ __forceinline__ bool tap_sums(int nch, int ne, int nsp, int k, long first, long stride,
+                                         const float2 *__restrict__ gP,
+                                         const char2 *__restrict__ iq, double (&out)[NT][VEC])
 {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
+    Sum acc[NT][VEC];
+    const long nruns = (long)ne * ((nsp + TG_RUN - 1) / TG_RUN);
+    const long spec = (long)ne * nch;
+    for (long t = first; t < nruns; t += stride) {
+        const int run = (int)(t / ne), e = (int)(t - (long)run * ne);
+        const int s0 = run * TG_RUN, s1 = min(nsp, s0 + TG_RUN);
+        const float2 *g = gP + (long)s0 * spec + (long)e * nch + k;
+        const char2 *x = iq + (long)s0 * spec + (long)e * nch + k;
+        float xr[NT][VEC], xi[NT][VEC];  // spectrum s in slot (s - s0) % NT
+#pragma unroll
+        for (int i = 0; i < NT - 1; i++) load_iq<VEC>(x + i * spec, xr[i], xi[i]);
+        for (int s = s0; s < s1; s += NT) {
+#pragma unroll
+            for (int u = 0; u < NT; u++) {
+                if (s + u < s1) {
+                    float2 gv[VEC];
+                    load_c64<VEC>(g + (long)(s + u - s0) * spec, gv);
+                    load_iq<VEC>(x + (long)(s + u - s0 + NT - 1) * spec, xr[(u + NT - 1) % NT],
+                                 xi[(u + NT - 1) % NT]);
+#pragma unroll
+                    for (int i = 0; i < NT; i++)
+#pragma unroll
+                        for (int v = 0; v < VEC; v++) {
+                            acc[i][v].add(gv[v].x, xr[(u + i) % NT][v]);
+                            acc[i][v].add(gv[v].y, xi[(u + i) % NT][v]);
+                        }
+                }
+            }
+        }
+    }
+    bool ok = true;
+#pragma unroll
+    for (int i = 0; i < NT; i++)
+#pragma unroll
+        for (int v = 0; v < VEC; v++) {
+            ok = ok && acc[i][v].finite();
+            out[i][v] = acc[i][v].value();
+        }
+    return ok;
+}
+
+template <int NT, int VEC>
+__global__ void __launch_bounds__(32 * TG_PH)
+    pfb_tap_grad_all_kernel(int nch, int ne, int nsp, int nsplit, const float2 *__restrict__ gP,
+                            const char2 *__restrict__ iq, double *__restrict__ part)
+{
+    __shared__ double red[TG_PH][32 * VEC];
+    const int k = (blockIdx.x * 32 + threadIdx.x) * VEC;
+    const int ph = threadIdx.y, p = blockIdx.y;
+    const long first = (long)p * TG_PH + ph, stride = (long)nsplit * TG_PH;
+    double sum[NT][VEC] = {};
+    if (k < nch && !tap_sums<NT, VEC, Sum2>(nch, ne, nsp, k, first, stride, gP, iq, sum))
+        tap_sums<NT, VEC, SumD>(nch, ne, nsp, k, first, stride, gP, iq, sum);
+    const int tid = ph * 32 + threadIdx.x;
+#pragma unroll
+    for (int i = 0; i < NT; i++) {
+#pragma unroll
+        for (int v = 0; v < VEC; v++) red[ph][threadIdx.x * VEC + v] = sum[i][v];
+        __syncthreads();
+        const int kk = blockIdx.x * 32 * VEC + tid;
+        if (tid < 32 * VEC && kk < nch) {
+            double acc = red[0][tid];
+            for (int q = 1; q < TG_PH; q++) acc += red[q][tid];
+            part[((long)p * NT + i) * nch + kk] = acc;
+        }
+        __syncthreads();
+    }
+}
+
+// gW[i][k] = sum_p part[p][i][k] (deterministic): eight interleaved partial
+// sums of 32 outputs per block, added in a fixed order.
+__global__ void __launch_bounds__(256)
+    pfb_tap_grad_reduce_kernel(int n, int nsplit, const double *__restrict__ part,
+                               float *__restrict__ gW)
+{
+    __shared__ double red[8][32];
+    const int j = blockIdx.x * 32 + threadIdx.x;
     double acc = 0.0;
-    for (int p = 0; p < nsplit; p++) acc += part[(long)p * n + j];
-    gW[j] = (float)acc;
+    if (j < n)
+        for (int p = threadIdx.y; p < nsplit; p += 8) acc += part[(long)p * n + j];
+    red[threadIdx.y][threadIdx.x] = acc;
+    __syncthreads();
+    if (threadIdx.y == 0 && j < n) {
+        for (int q = 1; q < 8; q++) acc += red[q][threadIdx.x];
+        gW[j] = (float)acc;
+    }
 }
 
 }  // namespace mdt
@@ -209,9 +416,19 @@ MDT_API mdt_status mdt_apply_gains(int ne, int nch, int nsp, const void *X, cons
 {
     if (!X || !gains || !Y || ne < 1 || nch < 1 || nsp < 1)
         return mdt::invalid("apply_gains: bad arguments");
-    const long n = (long)nch * nsp * ne;
-    mdt::apply_gains_kernel<<<(unsigned)mdt::cdiv(n, 256), 256, 0, stream>>>(
-        n, ne, nsp, (const float2 *)X, (const float2 *)gains, (float2 *)Y);
+    // 16-byte vectors need an even NE (every row and gain pair then starts on one)
+    const bool v2 = ne % 2 == 0 && (((uintptr_t)X | (uintptr_t)gains | (uintptr_t)Y) & 15) == 0;
+    const int vec = v2 ? 2 : 1;
+    const long per = (long)nsp * ne / vec;
+    const dim3 grid((unsigned)mdt::cdiv(per, mdt::AG_THREADS * mdt::AG_ITEMS),
+                    (unsigned)std::min(nch, 65535));
+    const int step = mdt::AG_THREADS * vec % ne;
+    if (v2)
+        mdt::apply_gains_kernel<2><<<grid, mdt::AG_THREADS, 0, stream>>>(
+            nch, ne, per, step, (const float2 *)X, (const float2 *)gains, (float2 *)Y);
+    else
+        mdt::apply_gains_kernel<1><<<grid, mdt::AG_THREADS, 0, stream>>>(
+            nch, ne, per, step, (const float2 *)X, (const float2 *)gains, (float2 *)Y);
     return mdt::launch_status("apply_gains_kernel");
 }
 
@@ -223,15 +440,23 @@ MDT_API mdt_status mdt_gain_adjoint(int ne, int nch, int nsp, const void *dY, co
         return mdt::invalid("gain_adjoint: bad arguments");
     if (dgains) {
         if (!X) return mdt::invalid("gain_adjoint: X is needed for the gain gradient");
-        mdt::gain_grad_kernel<<<(unsigned)mdt::cdiv((long)nch * ne, 32), dim3(32, 8), 0, stream>>>(
-            ne, nch, nsp, (const float2 *)dY, (const float2 *)X, (float2 *)dgains);
+        // 16-byte loads need an even NE (every row then starts on one)
+        const bool v2 = ne % 2 == 0 && (((uintptr_t)dY | (uintptr_t)X) & 15) == 0;
+        const dim3 block(32, mdt::GG_PH);
+        const unsigned blocks = (unsigned)mdt::cdiv((long)nch * (ne / (v2 ? 2 : 1)), 32);
+        if (v2)
+            mdt::gain_grad_kernel<2><<<blocks, block, 0, stream>>>(
+                ne, nch, nsp, (const float2 *)dY, (const float2 *)X, (float2 *)dgains);
+        else
+            mdt::gain_grad_kernel<1><<<blocks, block, 0, stream>>>(
+                ne, nch, nsp, (const float2 *)dY, (const float2 *)X, (float2 *)dgains);
         mdt_status st = mdt::launch_status("gain_grad_kernel");
         if (st != MDT_SUCCESS) return st;
     }
     if (dF) {
         const long rows = (long)nsp * ne;
-        dim3 grid((unsigned)mdt::cdiv(rows, 32), (unsigned)mdt::cdiv(nch, 32));
-        mdt::fout_adjoint_kernel<<<grid, dim3(32, 8), 0, stream>>>(
+        dim3 grid((unsigned)mdt::cdiv(rows, mdt::FA_T), (unsigned)mdt::cdiv(nch, mdt::FA_T));
+        mdt::fout_adjoint_kernel<<<grid, dim3(32, 16), 0, stream>>>(
             ne, nch, rows, (const float2 *)dY, (const float2 *)gains, (float2 *)dF);
         return mdt::launch_status("fout_adjoint_kernel");
     }
@@ -251,13 +476,27 @@ MDT_API mdt_status mdt_pfb_tap_grad(int ne, int nch, int ntaps, int nsp, const v
         return mdt::invalid("pfb_tap_grad: workspace must hold Ntaps*Nch doubles");
     mdt_status st;
     if (ntaps == 4 || ntaps == 8) {
-        dim3 grid((unsigned)mdt::cdiv(nch, 128), (unsigned)nsplit);
-        if (ntaps == 4)
-            mdt::pfb_tap_grad_all_kernel<4><<<grid, 128, 0, stream>>>(
+        // two channels per thread (16-byte gradients, 4-byte samples) where Nch is
+        // even and the buffers are aligned for it
+        const bool v2 = nch % 2 == 0 && ((uintptr_t)gradP & 15) == 0 && ((uintptr_t)iq & 3) == 0;
+        const long runs = (long)ne * mdt::cdiv(nsp, mdt::TG_RUN);
+        // two blocks of 16 warps fit an SM: as many splits as fill the GPU once
+        // (64 splits, 1.7 waves at Nch 512: 296 us against 265)
+        const long once = 2L * mdt::sm_count() / mdt::cdiv(nch, 32 * (v2 ? 2 : 1));
+        nsplit = (int)std::max<long>(1, std::min<long>(std::min<long>(nsplit, once),
+                                                       mdt::cdiv(runs, mdt::TG_PH)));
+        auto launch = [&](auto kern, int vec) {
+            const dim3 grid((unsigned)mdt::cdiv(nch, 32 * vec), (unsigned)nsplit);
+            kern<<<grid, dim3(32, mdt::TG_PH), 0, stream>>>(
                 nch, ne, nsp, nsplit, (const float2 *)gradP, (const char2 *)iq, (double *)workspace);
-        else
-            mdt::pfb_tap_grad_all_kernel<8><<<grid, 128, 0, stream>>>(
-                nch, ne, nsp, nsplit, (const float2 *)gradP, (const char2 *)iq, (double *)workspace);
+        };
+        if (ntaps == 4) {
+            if (v2) launch(mdt::pfb_tap_grad_all_kernel<4, 2>, 2);
+            else launch(mdt::pfb_tap_grad_all_kernel<4, 1>, 1);
+        } else {
+            if (v2) launch(mdt::pfb_tap_grad_all_kernel<8, 2>, 2);
+            else launch(mdt::pfb_tap_grad_all_kernel<8, 1>, 1);
+        }
         st = mdt::launch_status("pfb_tap_grad_all_kernel");
     } else {
         dim3 grid((unsigned)mdt::cdiv(nch, 128), (unsigned)ntaps, (unsigned)nsplit);
@@ -267,7 +506,7 @@ MDT_API mdt_status mdt_pfb_tap_grad(int ne, int nch, int ntaps, int nsp, const v
         st = mdt::launch_status("pfb_tap_grad_partial_kernel");
     }
     if (st != MDT_SUCCESS) return st;
-    mdt::pfb_tap_grad_reduce_kernel<<<(unsigned)mdt::cdiv(n, 256), 256, 0, stream>>>(
+    mdt::pfb_tap_grad_reduce_kernel<<<(unsigned)mdt::cdiv(n, 32), dim3(32, 8), 0, stream>>>(
         (int)n, nsplit, (const double *)workspace, gradW);
     return mdt::launch_status("pfb_tap_grad_reduce_kernel");
 }
