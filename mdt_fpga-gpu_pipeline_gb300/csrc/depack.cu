@@ -99,36 +99,173 @@ __global__ void depacketise_kernel(DepackGeom g, const unsigned char *__restrict
     }
 }
 
-// One thread per (station, SNAP, slot): zero-fill slots that never arrived,
-// count them, clear the arrival counts.
+// The same for packets whose 32-sample runs fit a warp's staging buffer: one
+// warp per packet, DP_PER packets per warp.  Payload words are copied
+// contiguously (WB = 16 bytes where the packets' alignment allows it, else 4)
+// into one of the warp's two buffers with cp.async, the next packet's before
+// this one's header is looked at, and written with the lanes along the samples
+// of one input, i.e. along channels.  The counters are summed per block and
+// added once (one atomic per packet on the same counter serialises in L2).
+// Bound by HBM: 8 + 8 (int32) or 2 + 2 (int8) bytes a sample.  38 inputs, 1024
+// channels and spectra, 28 samples a packet, int32: 123 us (5.2 TB/s) against
+// 205 us with a block per packet and strided 8-byte reads; without the second
+// buffer 141 us.
+constexpr int DP_WARPS = 4, DP_PER = 8;
+constexpr int DP_BUF = 4096;  // bytes of a staging buffer
+
+template <int WB>
+__device__ __forceinline__ void copy_words(unsigned char *dst, const unsigned char *src, int words,
+                                           int lane)
+{
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+    for (int w = lane; w < words; w += 32)
+        if constexpr (WB == 16)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d + 16 * w),
+                         "l"(src + 16 * w)
+                         : "memory");
+        else
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d + 4 * w),
+                         "l"(src + 4 * w)
+                         : "memory");
+    asm volatile("cp.async.commit_group;" ::: "memory");
+}
+
+template <int WB>
+__global__ void __launch_bounds__(32 * DP_WARPS)
+    depacketise_warp_kernel(DepackGeom g, int maxn, const unsigned char *__restrict__ pkts,
+                            int npackets, void *__restrict__ out, unsigned int *__restrict__ seen,
+                            mdt_depack_stats *__restrict__ stats)
+{
+    __shared__ __align__(16) unsigned char sbuf[DP_WARPS][2][DP_BUF];
+    __shared__ unsigned int s_cnt[4];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x < 4) s_cnt[threadIdx.x] = 0;
+    __syncthreads();
+    const int per = g.bits == 32 ? 8 : 2;  // bytes of a sample
+    const long long wlen = (long long)g.nspectra * g.nch;
+    // the first run of a packet, sized for the widest SNAP (inside the packet
+    // whatever its SNAP is: packet_bytes holds the widest payload)
+    const int lead = (min(32, g.sper) * maxn * per + WB - 1) / WB;
+    const long pk0 = (long)blockIdx.x * (DP_PER * DP_WARPS) + warp;
+    const unsigned char *pay = pkts + 4 * g.hdr_words;
+    if (pk0 < npackets) copy_words<WB>(sbuf[warp][0], pay + pk0 * g.pkt_bytes, lead, lane);
+    for (int m = 0; m < DP_PER; m++) {
+        const long pk = pk0 + (long)m * DP_WARPS;
+        if (pk >= npackets) break;
+        unsigned char *buf = sbuf[warp][m & 1];
+        // the packet after this one (an empty group when there is none)
+        const bool more = m + 1 < DP_PER && pk + DP_WARPS < npackets;
+        copy_words<WB>(sbuf[warp][(m + 1) & 1], pay + (pk + DP_WARPS) * g.pkt_bytes,
+                       more ? lead : 0, lane);
+        const uint32_t *hdr = (const uint32_t *)(pkts + pk * g.pkt_bytes);
+        const uint32_t station = __ldg(hdr), snap = __ldg(hdr + 1), counter = __ldg(hdr + 2);
+        const long long slot = (long long)counter - g.c0;
+        if (snap >= (uint32_t)g.nsnap || station >= (uint32_t)g.nstation ||
+            (long)station * g.ips + g.snap_off[snap] + g.snap_n[snap] > g.ne) {
+            if (lane == 0) atomicAdd(&s_cnt[2], 1u);
+            continue;
+        }
+        if (slot < 0 || slot >= g.nslots) {
+            if (lane == 0) atomicAdd(&s_cnt[1], 1u);
+            continue;
+        }
+        if (lane == 0) {
+            const unsigned int prev =
+                atomicAdd(&seen[((long)station * g.nsnap + snap) * g.nslots + slot], 1u);
+            if (prev) atomicAdd(&s_cnt[3], 1u);
+            atomicAdd(&s_cnt[0], 1u);
+        }
+        const int nin = g.snap_n[snap];
+        const long elem0 = (long)station * g.ips + g.snap_off[snap];
+        const long long first = (long long)counter * g.sper - g.sample0;
+        for (int i0 = 0; i0 < g.sper; i0 += 32) {
+            // samples i0 .. i0 + 31 of every input are contiguous; a run starts
+            // on a multiple of 32 samples, so on a 16-byte boundary of the payload
+            const int ns = min(32, g.sper - i0);
+            if (i0) {
+                copy_words<WB>(buf, pay + pk * g.pkt_bytes + (long)i0 * nin * per,
+                               (ns * nin * per + WB - 1) / WB, lane);
+                asm volatile("cp.async.wait_group 0;" ::: "memory");
+            } else {
+                asm volatile("cp.async.wait_group 1;" ::: "memory");
+            }
+            __syncwarp();
+            const long long s = first + i0 + lane;
+            if (lane < ns && s >= 0 && s < wlen) {
+                // 32-bit division wherever the window's sample index fits
+                const long spec = wlen >> 32 ? (long)(s / g.nch)
+                                             : (long)((unsigned)s / (unsigned)g.nch);
+                const long o = (spec * g.ne + elem0) * g.nch + (long)(s - (long long)spec * g.nch);
+                if (g.bits == 32) {
+                    const uint2 *v = (const uint2 *)buf + lane * nin;
+                    float2 *dst = (float2 *)out + o;
+#pragma unroll 2
+                    for (int j = 0; j < nin; j++, dst += g.nch)
+                        *dst = make_float2(fixed19_to_float(v[j].x), fixed19_to_float(v[j].y));
+                } else {
+                    const char2 *v = (const char2 *)buf + lane * nin;
+                    char2 *dst = (char2 *)out + o;
+#pragma unroll 2
+                    for (int j = 0; j < nin; j++, dst += g.nch) *dst = v[j];
+                }
+            }
+            __syncwarp();
+        }
+    }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    if (threadIdx.x < 4 && s_cnt[threadIdx.x]) {
+        unsigned long long *c = threadIdx.x == 0   ? &stats->accepted
+                                : threadIdx.x == 1 ? &stats->outside
+                                : threadIdx.x == 2 ? &stats->bad
+                                                   : &stats->duplicate;
+        atomicAdd(c, (unsigned long long)s_cnt[threadIdx.x]);
+    }
+}
+
+// One thread per (station, SNAP, slot) looks for slots that never arrived and
+// clears the arrival counts; its warp then zero-fills the missing slots it
+// found one after another, all lanes on one slot (lanes along the samples):
+// one slot per thread left the kernel waiting for its slowest thread (15 us
+// against 3.4 with 0.1 % of the packets lost).
 __global__ void depack_finish_kernel(DepackGeom g, void *__restrict__ out,
                                      unsigned int *__restrict__ seen,
                                      mdt_depack_stats *__restrict__ stats)
 {
     const long t = (long)blockIdx.x * blockDim.x + threadIdx.x;
     const long ngrp = (long)g.nstation * g.nsnap;
-    if (t >= ngrp * g.nslots) return;
-    const long grp = t / g.nslots, slot = t - grp * g.nslots;
-    const int station = (int)(grp / g.nsnap), snap = (int)(grp - (long)station * g.nsnap);
-    const long elem0 = (long)station * g.ips + g.snap_off[snap];
-    const int nin = g.snap_n[snap];
-    const unsigned int n = seen[t];
-    seen[t] = 0;
-    if (n || elem0 + nin > g.ne || nin == 0) return;
-    atomicAdd(&stats->missing, 1ull);
-    const long long first = (g.c0 + slot) * g.sper - g.sample0;
+    bool miss = false;
+    if (t < ngrp * g.nslots) {
+        const long grp = t / g.nslots;
+        const int station = (int)(grp / g.nsnap), snap = (int)(grp - (long)station * g.nsnap);
+        const unsigned int n = seen[t];
+        if (n) seen[t] = 0;
+        miss = !n && g.snap_n[snap] > 0 &&
+               (long)station * g.ips + g.snap_off[snap] + g.snap_n[snap] <= g.ne;
+    }
+    unsigned int todo = __ballot_sync(0xffffffffu, miss);
+    if (!todo) return;
+    const int lane = threadIdx.x & 31;
+    if (lane == 0) atomicAdd(&stats->missing, (unsigned long long)__popc(todo));
     const long long wlen = (long long)g.nspectra * g.nch;
-    for (int i = 0; i < g.sper; i++) {
-        const long long s = first + i;
-        if (s < 0 || s >= wlen) continue;
-        const long long spec = s / g.nch;
-        const int chan = (int)(s - spec * g.nch);
-        for (int j = 0; j < nin; j++) {
-            const long o = ((long)spec * g.ne + elem0 + j) * g.nch + chan;
-            if (g.bits == 32)
-                ((float2 *)out)[o] = make_float2(0.f, 0.f);
-            else
-                ((char2 *)out)[o] = make_char2(0, 0);
+    for (; todo; todo &= todo - 1) {
+        const long tm = t - lane + (__ffs(todo) - 1);
+        const long grp = tm / g.nslots, slot = tm - grp * g.nslots;
+        const int station = (int)(grp / g.nsnap), snap = (int)(grp - (long)station * g.nsnap);
+        const long elem0 = (long)station * g.ips + g.snap_off[snap];
+        const int nin = g.snap_n[snap];
+        const long long first = (g.c0 + slot) * g.sper - g.sample0;
+        for (int i = lane; i < g.sper; i += 32) {
+            const long long s = first + i;
+            if (s < 0 || s >= wlen) continue;
+            const long long spec = s / g.nch;
+            const long o = ((long)spec * g.ne + elem0) * g.nch + (long)(s - spec * g.nch);
+            for (int j = 0; j < nin; j++) {
+                if (g.bits == 32)
+                    ((float2 *)out)[o + (long)j * g.nch] = make_float2(0.f, 0.f);
+                else
+                    ((char2 *)out)[o + (long)j * g.nch] = make_char2(0, 0);
+            }
         }
     }
 }
@@ -202,6 +339,24 @@ MDT_API mdt_status mdt_depacketise(const mdt_packet_format *fmt, const void *pac
     if (npackets == 0) return MDT_SUCCESS;
     if (((uintptr_t)packets & 3) || ((uintptr_t)out & (fmt->sample_bits == 32 ? 7 : 1)))
         return mdt::invalid("depacketise: misaligned packets or output");
+    // A warp per packet while 32 samples of the widest SNAP fit its staging
+    // buffer (16 inputs of int32, 64 of int8); wider SNAPs take a block per packet.
+    int maxn = 0;
+    for (int k = 0; k < fmt->nsnap; k++) maxn = std::max(maxn, fmt->inputs_per_snap[k]);
+    if ((long)maxn * 32 * (fmt->sample_bits == 32 ? 8 : 2) <= mdt::DP_BUF) {
+        const unsigned blocks = (unsigned)mdt::cdiv(npackets, mdt::DP_WARPS * mdt::DP_PER);
+        // 16-byte reads where every payload starts on a 16-byte boundary and the
+        // packet stride keeps the last read inside the packet
+        const bool wide = (((uintptr_t)packets | (uintptr_t)fmt->packet_bytes |
+                            (uintptr_t)(4L * fmt->words_header)) & 15) == 0;
+        if (wide)
+            mdt::depacketise_warp_kernel<16><<<blocks, 32 * mdt::DP_WARPS, 0, stream>>>(
+                g, maxn, (const unsigned char *)packets, npackets, out, seen, stats);
+        else
+            mdt::depacketise_warp_kernel<4><<<blocks, 32 * mdt::DP_WARPS, 0, stream>>>(
+                g, maxn, (const unsigned char *)packets, npackets, out, seen, stats);
+        return mdt::launch_status("depacketise_warp_kernel");
+    }
     mdt::depacketise_kernel<<<(unsigned)npackets, 128, 0, stream>>>(
         g, (const unsigned char *)packets, out, seen, stats);
     return mdt::launch_status("depacketise_kernel");
