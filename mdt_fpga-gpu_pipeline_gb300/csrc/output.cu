@@ -23,44 +23,71 @@
 namespace mdt {
 
 // Baseline index of (j, p, k, q), k >= j, q >= p, in the reference's loop order.
-__host__ __device__ __forceinline__ long baseline_index(long nel, long np, long j, long p, long k,
-                                                        long q)
+// In I = unsigned, exact while Nelements * Npols <= 65535 (fewer than 2^32 baselines).
+template <class I>
+__host__ __device__ __forceinline__ I baseline_index(I nel, I np, I j, I p, I k, I q)
 {
-    const long T = np * (np + 1) / 2;
+    const I T = np * (np + 1) / 2;
     return T * (j * nel - j * (j - 1) / 2) + (nel - j) * (p * np - p * (p - 1) / 2) +
            (k - j) * (np - p) + (q - p);
 }
 
-// Block: one column c = k*Np + q, 32 rows r, 32 channels.  Reads run along r
-// (contiguous in V), writes along z (contiguous in out).
-__global__ void format_baselines_kernel(int nel, int np, int nch, int shift,
-                                        const float2 *__restrict__ V, float2 *__restrict__ out)
+// Block: one column c = k*Np + q, 32 rows r <= c, FB_Z channels.  Reads run
+// along r (contiguous in V), writes along z (contiguous in out), 256 bytes a
+// warp each way.  Bound by HBM (8 bytes read and 8 written per baseline and
+// channel): FB_Z = 64 keeps eight independent loads per thread in flight, the
+// grid holds only tiles on or below the diagonal, and four lanes of a warp form
+// its rows' baseline indices.  NE=256 (two polarisations), Nch=1024: 113 us
+// (3.6 TB/s of the baselines' bytes, more with the columns' unused rows in the
+// same sectors); 32 x 32 tiles with an index per row and thread took 262 us.
+constexpr int FB_Z = 64;
+
+__global__ void __launch_bounds__(256)
+    format_baselines_kernel(int nel, int np, int nch, int shift, const float2 *__restrict__ V,
+                            float2 *__restrict__ out)
 {
-    __shared__ float2 t[32][33];
+    __shared__ float2 t[FB_Z][33];
     const int ne = nel * np;
-    const int c = blockIdx.x;
-    const int r0 = blockIdx.y * 32;
-    const int z0 = blockIdx.z * 32;
+    // blockIdx.x = 32 * (ct (ct + 1) / 2 + rt) + (c mod 32): row tiles rt <= ct
+    const int pair = (int)(blockIdx.x >> 5);
+    int ct = (int)((sqrtf(8.0f * pair + 1.0f) - 1.0f) * 0.5f);
+    while ((ct + 1) * (ct + 2) / 2 <= pair) ct++;
+    while (ct * (ct + 1) / 2 > pair) ct--;
+    const int c = ct * 32 + (int)(blockIdx.x & 31), r0 = (pair - ct * (ct + 1) / 2) * 32;
+    if (c >= ne) return;
+    const int z0 = blockIdx.y * FB_Z;
     const int k = c / np, q = c - k * np;
-    if (r0 > c) return;  // rows past the column hold no baseline (k >= j needs r <= c)
-    for (int y = threadIdx.y; y < 32; y += blockDim.y) {
-        const int z = z0 + y, r = r0 + threadIdx.x;
-        float2 v = make_float2(0.f, 0.f);
-        if (z < nch && r < ne) {
-            const int i = shift ? (z + nch / 2) % nch : z;
-            v = V[((long)i * ne + c) * ne + r];
-        }
-        t[y][threadIdx.x] = v;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int r = r0 + lane;
+    const float2 *src = V + (long)c * ne + r;
+    const long cstride = (long)ne * ne;
+#pragma unroll
+    for (int y = 0; y < FB_Z / 8; y++) {
+        const int z = z0 + warp + 8 * y;
+        int i = shift ? z + nch / 2 : z;
+        if (i >= nch) i -= nch;
+        // rows past the column hold no baseline (k >= j needs r < (k + 1) Np)
+        if (z < nch && r < ne && r / np <= k) t[warp + 8 * y][lane] = __ldg(src + i * cstride);
+    }
+    // lanes 0..3 form the baseline indices of the warp's rows warp + 8 * lane
+    // (0xffffffff: the row holds no baseline of this column)
+    unsigned mine = 0xffffffffu;
+    if (lane < 4) {
+        const int row = r0 + warp + 8 * lane, j = row / np, pp = row - j * np;
+        if (row < ne && k >= j && q >= pp) mine = baseline_index<unsigned>(nel, np, j, pp, k, q);
     }
     __syncthreads();
-    const long nel_l = nel;
-    for (int y = threadIdx.y; y < 32; y += blockDim.y) {
-        const int r = r0 + y, z = z0 + threadIdx.x;
-        if (r >= ne || z >= nch) continue;
-        const int j = r / np, p = r - j * np;
-        if (k < j || q < p) continue;
-        const long bl = baseline_index(nel_l, np, j, p, k, q);
-        out[bl * nch + z] = t[threadIdx.x][y];
+#pragma unroll
+    for (int y = 0; y < 4; y++) {
+        const int rr = warp + 8 * y;
+        const unsigned bl = __shfl_sync(0xffffffffu, mine, y);
+        if (bl == 0xffffffffu) continue;
+        float2 *dst = out + (long)bl * nch;
+#pragma unroll
+        for (int h = 0; h < FB_Z / 32; h++) {
+            const int z = z0 + 32 * h + lane;
+            if (z < nch) dst[z] = t[32 * h + lane][rr];
+        }
     }
 }
 
@@ -162,9 +189,10 @@ MDT_API mdt_status mdt_format_baselines(int nelements, int npols, int nch, const
         return mdt::invalid("format_baselines: bad arguments");
     if (fftshift && (nch & 1)) return mdt::invalid("format_baselines: fftshift needs even Nch");
     const int ne = nelements * npols;
-    dim3 grid((unsigned)ne, (unsigned)mdt::cdiv(ne, 32), (unsigned)mdt::cdiv(nch, 32));
-    if (grid.z > 65535) return mdt::invalid("format_baselines: Nch too large");
-    mdt::format_baselines_kernel<<<grid, dim3(32, 8), 0, stream>>>(
+    if (mdt::cdiv(nch, 32) > 65535) return mdt::invalid("format_baselines: Nch too large");
+    const long nt = mdt::cdiv(ne, 32);
+    dim3 grid((unsigned)(nt * (nt + 1) / 2 * 32), (unsigned)mdt::cdiv(nch, mdt::FB_Z));
+    mdt::format_baselines_kernel<<<grid, 256, 0, stream>>>(
         nelements, npols, nch, fftshift ? 1 : 0, (const float2 *)vis, (float2 *)out);
     return mdt::launch_status("format_baselines_kernel");
 }
