@@ -61,10 +61,11 @@ def test_format_tiles(mdt, cuda, nel, npol, nch):
     assert np.array_equal(out.cpu().numpy().view(np.uint64), want.view(np.uint64))
 
 
-# 8216 blocks of 1024 threads: runs of eight spectra, the last of three
+# enough blocks for runs of 16 spectra (the last of 3) and of 32 (the last of 11)
+@pytest.mark.parametrize("nsp", [2563, 5003])
 @pytest.mark.parametrize("ntaps", [4, 8, 16, 5])
-def test_pps_runs(mdt, cuda, oracle, ntaps):
-    nch, ne, nsp = 64, 8, 1027
+def test_pps_runs(mdt, cuda, oracle, ntaps, nsp):
+    nch, ne = 64, 8
     rng = np.random.default_rng(ntaps)
     x = crandn(rng, nsp + ntaps - 1, ne, nch).astype(np.complex64)
     w = rng.standard_normal(ntaps * nch).astype(np.float32)
