@@ -155,3 +155,20 @@ def test_gain_sums_and_rows(mdt, cuda, ne, nch, nsp, off):
     assert not np.isfinite(got[1, 0]) and np.isinf(got[1, 0].real)
     got[1, 0] = 0
     assert np.all(np.isfinite(got))
+
+
+# one chunk of 64 elements kept over several tiles of 64 spectra, a second block of
+# tiles, and two chunks
+@pytest.mark.parametrize("ne,nch,nsp", [(64, 2, 300), (65, 1, 257), (7, 3, 520)])
+def test_xengine_adjoint_tiles(mdt, cuda, ne, nch, nsp):
+    rng = np.random.default_rng(ne + nsp)
+    G = crandn(rng, nch, ne, ne).astype(np.complex64)
+    Y = crandn(rng, nch, nsp, ne).astype(np.complex64)
+    dY = torch.full((nch, nsp, ne), float("nan"), dtype=torch.complex64, device="cuda")
+    mdt.xengine_adjoint_f32(ne, nch, nsp, dev(G), dev(Y), dY, 0.5)
+    Gm = np.transpose(G.astype(np.complex128), (0, 2, 1))
+    H = Gm + np.conj(np.transpose(Gm, (0, 2, 1)))
+    want = 0.5 * np.einsum("crq,csq->csr", H, Y.astype(np.complex128))
+    # four multiply-adds per q: under 4 NE 2^-24 of the sum of magnitudes
+    mag = 0.5 * np.einsum("crq,csq->csr", np.abs(H), np.abs(Y))
+    assert np.all(np.abs(dY.cpu().numpy() - want) <= 4 * ne * 2.0 ** -24 * mag)
