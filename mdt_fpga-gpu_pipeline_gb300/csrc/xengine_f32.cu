@@ -1,0 +1,467 @@
+// xengine_f32.cu -- FP32 Hermitian X-engine on the tensor cores: per channel c
+//   V_c = alpha * X_c X_c^H (+ beta V_c)
+// on the lower triangle, mirrored; the reference's cublasCgemmBatched call
+// (OP_N, OP_C, A == B, alpha = 1/Nspectra, beta = 0;
+// MDT_OneStation_client.cu:1128, :656-660, :683-686).
+//
+// Arithmetic.  Over a stage of 64 spectra an element's samples are scaled by a
+// power of two that brings the largest component to [1024, 2048) and split into
+// an integer h and the rest l in f16: x s = h + l, |l| <= 1/2, which keeps 23
+// bits below the largest component.  A product of two samples is
+//   (x s)(y t) = h h' + (h l' + l h' + l l'),
+// exact f16 products all.  The h h' sum is kept apart from the others: it is a
+// sum of integers, exact in FP32 below 2^24 (about its size for noise-like samples;
+// beyond, it loses a unit in the last place).  That matters because the tensor
+// core truncates when it adds to its accumulator: sums with fractions lose half a
+// unit per step, always towards zero (f16 pairs split by value: autocorrelations
+// 2.3e-7 low after 64 spectra).  The stage's sums go to FP32 registers, XF_FLUSH
+// stages at a time and then to a second level, so that a visibility of 1000
+// spectra is rounded about ten times, not a thousand times.
+// Relative error of V against 64-bit sums of the same FP32 samples (normal
+// noise), here and by FP32 multiply-adds in spectrum order (the SIMT kernel):
+//   NE=10, Nsp=1000: 5.8e-8, 9.2e-8;   NE=40, Nsp=512: 7.1e-8, 2.4e-7;
+//   NE=40, Nsp=4096: 6.0e-8, 6.2e-7;   NE=256, Nsp=2048: 7.9e-8, 8.8e-7.
+//
+// Samples or products that are not finite make the affected sums NaN; every
+// visibility that comes out non-finite is formed again by FP32 multiply-adds
+// over its two elements, so infinities and NaN appear as that sum gives
+// them.  A block whose waits gave up (each is bounded) forms its whole tile
+// that way.
+//
+// Layout of the products: re and im of an element are separate rows of one real
+// operand Z (2 nb rows, nb = elements rounded up to 8), and D = Z Z^T holds
+//   Re V_rq = D[re r][re q] + D[im r][im q],  Im V_rq = D[im r][re q] - D[re r][im q],
+// four real products per pair and no product formed twice.  M = 128 rows are 64
+// elements of one channel, or, so that small arrays fill the instruction and
+// share its latency, 32 elements of two channels or 16 of four (the products
+// between channels are ignored).  Larger arrays are cut into 64 x 64 tiles.
+//
+// A block per SM: sixteen converting warps and an issuing one (issuing an MMA
+// holds the thread until the queue takes it).  Per stage a converting thread
+// loads eight samples of one element per operand, converts them into words of
+// the K-major 128-byte-swizzled operand, and adds the sums of an earlier stage from
+// tensor memory to its registers.  Two operand stages and two accumulator sets
+// alternate: while the tensor core works on stage k + 1, the warps drain stage k
+// and write stage k + 2 over its operands.
+//
+// What bounds it: an M = 128, K = 16 MMA takes 63 cycles for any N up to 128, so the
+// sixteen of a stage take 1000 of the 2200 to 3000 cycles that a stage takes; the
+// rest is the warps' chain of tensor-memory reads (about 300 cycles a batch under
+// MMAs), conversion and sample loads, one after the other.  Times, against the
+// SIMT kernel's: NE=256, Nch=1024, Nsp=2048 4.98 ms, 12.53; NE=64, Nch=512, Nsp=2048
+// 0.33, 0.70; NE=38, Nch=Nsp=1024 0.20, 0.28; NE=40, Nch=2048, Nsp=4096 1.35, 1.47;
+// NE=10, Nch=1024, Nsp=1000 0.058, 0.083.
+#include <algorithm>
+
+#include "tc_ptx.cuh"
+#include "xengine_f32.cuh"
+
+namespace mdt {
+
+constexpr int XF_WARPS = 16;                      // converting warps
+constexpr int XF_THREADS = 32 * (XF_WARPS + 1);   // and the issuing warp
+constexpr int XF_K = 64;                          // spectra per stage
+constexpr int XF_PLANE = 128 * 128;               // 128 rows of 64 f16
+constexpr int XF_OPERAND = 2 * XF_PLANE;          // h, l
+constexpr int XF_AHEAD = 3;                       // stages between L2 prefetch and load
+constexpr int XF_FLUSH = 8;                       // stages per first-level sum
+// Spectra from which the tensor cores are used.  Shorter sums round little in
+// FP32 multiply-adds (NE=10: 6.7e-8 at 64 spectra, 8.6e-8 at 250), there the split
+// is no closer to the 64-bit sums, and there is little time to gain.
+constexpr int XF_MIN_SPECTRA = 256;
+constexpr int XF_DS = 129;                        // floats per row of the exchanged sums
+constexpr size_t XF_D_BYTES = (size_t)128 * XF_DS * sizeof(float);
+constexpr size_t xf_smem(bool off)
+{
+    return 1024 + (size_t)2 * (off ? 2 : 1) * XF_OPERAND + XF_D_BYTES;
+}
+
+struct XfArgs {
+    int ne, nsp, npairs;
+    int nb;                      // operand rows of re (and of im) per channel
+    const float2 *X;             // base (when Xptrs == nullptr)
+    const float2 *const *Xptrs;  // per-channel operand pointers (cuBLAS shim)
+    long ld, xstride;
+    float2 *V;
+    float2 *const *Vptrs;
+    long ldv, vstride;
+    float2 alpha, beta;
+    int beta_zero;
+    long nbatch;
+};
+
+// Two floats as packed f16 (a in the low half), round to nearest even.
+__device__ __forceinline__ uint32_t f16x2(float2 v)
+{
+    uint32_t r;
+    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(v.y), "f"(v.x));
+    return r;
+}
+
+// V_rq by multiply-adds in spectrum order (results that are not finite).
+template <bool BLOCKED>
+__device__ __noinline__ float2 direct_product(const float2 *Xc, long ld, int nsp, int r, int q)
+{
+    float2 v = make_float2(0.f, 0.f);
+    for (int k = 0; k < nsp; k++) {
+        const float2 a = BLOCKED ? Xc[(long)(k >> 3) * ld + (long)r * 8 + (k & 7)] : Xc[(long)k * ld + r];
+        const float2 b = BLOCKED ? Xc[(long)(k >> 3) * ld + (long)q * 8 + (k & 7)] : Xc[(long)k * ld + q];
+        v.x = fmaf(a.x, b.x, v.x);
+        v.x = fmaf(a.y, b.y, v.x);
+        v.y = fmaf(a.y, b.x, v.y);
+        v.y = fmaf(-a.x, b.y, v.y);
+    }
+    return v;
+}
+
+// OFF: the grid holds tiles below the diagonal (NE > 64), with an operand of
+// their own for the columns.  SLOT: rows of M per channel (128, 64 or 32).
+// BLOCKED: operand X[(k/8)*ld + e*8 + k%8] (blocks of 8 spectra, the last one
+// zero-padded), else X[k*ld + e].
+template <bool OFF, int SLOT, bool BLOCKED>
+__global__ void __launch_bounds__(XF_THREADS, 1) xengine_f32_kernel(const XfArgs a)
+{
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    __shared__ uint64_t bars[4];  // full[2] (operands written), done[2] (products complete)
+    __shared__ uint32_t tmem_slot;
+    __shared__ int s_fail;
+    __shared__ __align__(16) float s_inv[4][2][64];  // [stage % 4][operand][element]: 1 / scale
+    constexpr int NSLOT = 128 / SLOT, EB = SLOT / 2;  // channels, and elements per channel
+    constexpr int STAGE = (OFF ? 2 : 1) * XF_OPERAND;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, tid = threadIdx.x;
+
+    const long ch0 = OFF ? blockIdx.x / a.npairs : (long)blockIdx.x * NSLOT;
+    int I = 0, J = 0;
+    if constexpr (OFF) {
+        const int p = (int)(blockIdx.x - ch0 * a.npairs);  // p = I (I + 1) / 2 + J
+        I = (int)((sqrtf(8.0f * p + 1.0f) - 1.0f) * 0.5f);
+        while ((I + 1) * (I + 2) / 2 <= p) I++;
+        while (I * (I + 1) / 2 > p) I--;
+        J = p - I * (I + 1) / 2;
+    }
+    const bool sep = OFF && I != J;  // columns have their own operand
+    const int r0 = I * 64, q0 = J * 64;
+    const int nr = min(EB, a.ne - r0), nq = min(EB, a.ne - q0);
+    const int nb = OFF ? 64 : a.nb;
+    const int nstage = (a.nsp + XF_K - 1) / XF_K;
+
+    if (tid == 0) {
+        for (int i = 0; i < 2; i++) {
+            tc::mbar_init(tc::smem_u32(&bars[i]), XF_WARPS);
+            tc::mbar_init(tc::smem_u32(&bars[2 + i]), 1);
+        }
+        s_fail = 0;
+        tc::fence_mbar_init();
+    }
+    if (warp == XF_WARPS) {
+        tc::tmem_alloc(tc::smem_u32(&tmem_slot), 512);
+        tc::tmem_relinquish();
+        tc::fence_before_sync();
+    }
+    __syncthreads();
+    tc::fence_after_sync();
+    const uint32_t tmem = tmem_slot;
+
+    if (warp == XF_WARPS) {
+        if (lane == 0) {
+            // ---------------- MMA issuer: h h' to columns 0..127 of the stage's set,
+            // the products with l to columns 128..255
+            const int N = (NSLOT - 1) * SLOT + 2 * nb;
+            const uint32_t id = tc::idesc_f16(N, 0, 0);
+            bool ok = true;
+            for (int k = 0; k < nstage && ok; k++) {
+                const int s = k & 1;
+                ok = tc::mbar_wait(tc::smem_u32(&bars[s]), (k >> 1) & 1);
+                if (!ok) break;
+                tc::fence_after_sync();
+                const uint32_t sa = tc::smem_u32(smem + (size_t)s * STAGE);
+                const uint64_t ad = tc::sw128_kmajor_desc(sa);
+                const uint64_t bd = tc::sw128_kmajor_desc(sep ? sa + XF_OPERAND : sa);
+                const uint32_t d = tmem + (uint32_t)(s * 256);
+                constexpr uint64_t L = XF_PLANE >> 4;
+#pragma unroll
+                for (int j = 0; j < 4; j++) {  // 16 spectra each
+                    tc::mma_f16(d, ad + 2 * j, bd + 2 * j, id, j > 0);
+                    tc::mma_f16(d + 128, ad + L + 2 * j, bd + L + 2 * j, id, j > 0);
+                    tc::mma_f16(d + 128, ad + 2 * j, bd + L + 2 * j, id, 1);
+                    tc::mma_f16(d + 128, ad + L + 2 * j, bd + 2 * j, id, 1);
+                }
+                tc::mma_commit(tc::smem_u32(&bars[2 + s]));
+            }
+            if (!ok) atomicExch(&s_fail, 1);
+        }
+        __syncwarp();
+    } else {
+        // ---------------- converting warps.  A thread takes element e of channel
+        // slot g and the spectra 8 (4 sg + i) + 2 p + {0, 1}, i < 4, of a stage: in
+        // the blocked layout four lanes (p) read 64 contiguous bytes, and a warp's
+        // 4-byte stores fall in 32 banks.
+        const int p = lane & 3, sg = (lane >> 2) & 1, el = warp * 4 + (lane >> 3);
+        const int e = el % EB, g = el / EB;
+        const bool liveA = ch0 + g < a.nbatch && e < nr, liveB = sep && e < nq;
+        const long ch = min(ch0 + g, a.nbatch - 1);
+        const float2 *Xc = a.Xptrs ? a.Xptrs[ch] : a.X + ch * a.xstride;
+        const float2 *xa = Xc + (BLOCKED ? (long)(r0 + e) * 8 : (long)(r0 + e));
+        const float2 *xb = Xc + (BLOCKED ? (long)(q0 + e) * 8 : (long)(q0 + e));
+        float2 re[4], im[4];  // the two spectra of run i
+        auto load = [&](const float2 *x, bool live, int k) {
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const int s = k * XF_K + 8 * (4 * sg + i);
+                if constexpr (BLOCKED) {
+                    const float4 v = live && s < a.nsp
+                                         ? __ldg(reinterpret_cast<const float4 *>(x + (long)(s >> 3) * a.ld) + p)
+                                         : make_float4(0.f, 0.f, 0.f, 0.f);
+                    re[i] = make_float2(v.x, v.z);
+                    im[i] = make_float2(v.y, v.w);
+                } else {
+                    const int s2 = s + 2 * p;
+                    const float2 u = live && s2 < a.nsp ? __ldg(x + (long)s2 * a.ld) : make_float2(0.f, 0.f);
+                    const float2 v = live && s2 + 1 < a.nsp ? __ldg(x + (long)(s2 + 1) * a.ld)
+                                                            : make_float2(0.f, 0.f);
+                    re[i] = make_float2(u.x, v.x);
+                    im[i] = make_float2(u.y, v.y);
+                }
+            }
+            // into L2, XF_AHEAD stages further on
+            if constexpr (BLOCKED) {
+                const int s = (k + XF_AHEAD) * XF_K + 8 * (4 * sg + p);
+                if (live && s < a.nsp && !(e & 1))
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(x + (long)(s >> 3) * a.ld));
+            } else {
+                const int s = (k + XF_AHEAD) * XF_K + 8 * (4 * sg + p) + 2 * (e & 3);
+                if (live && s < a.nsp) {
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(x + (long)s * a.ld));
+                    if (s + 1 < a.nsp)
+                        asm volatile("prefetch.global.L2 [%0];" ::"l"(x + (long)(s + 1) * a.ld));
+                }
+            }
+        };
+        auto convert = [&](int k, int op, bool live) {
+            // the eight lanes of an element agree on the scale
+            float m = 0.0f;
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                m = fmaxf(m, fmaxf(fabsf(re[i].x), fabsf(re[i].y)));
+                m = fmaxf(m, fmaxf(fabsf(im[i].x), fabsf(im[i].y)));
+            }
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+            // scale 2^(10 - exponent of m); at most 2^126, so that its inverse is normal
+            const int bs = min(127 + 10 + 127 - (int)(__float_as_uint(m) >> 23), 253);
+            const float sc = __uint_as_float((uint32_t)bs << 23);
+            if ((lane & 7) == 0) s_inv[k & 3][op][el] = __uint_as_float((uint32_t)(254 - bs) << 23);
+            if (!live) return;  // rows without an element feed sums that are never read
+            const float2 sc2 = make_float2(sc, sc);
+            const float2 big = make_float2(12582912.0f, 12582912.0f);  // 1.5 * 2^23: rounds to integers
+            const float2 nbig = make_float2(-12582912.0f, -12582912.0f);
+            uint8_t *st = smem + (size_t)(k & 1) * STAGE + (size_t)op * XF_OPERAND;
+#pragma unroll
+            for (int c = 0; c < 2; c++) {
+                const int row = g * SLOT + c * nb + e;
+                uint8_t *w = st + row * 128 + 4 * p;
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    const float2 x = c ? im[i] : re[i];
+                    const float2 h = __fadd2_rn(__ffma2_rn(x, sc2, big), nbig);
+                    const float2 l = __ffma2_rn(x, sc2, make_float2(-h.x, -h.y));
+                    const int at = ((4 * sg + i) ^ (row & 7)) << 4;
+                    *reinterpret_cast<uint32_t *>(w + at) = f16x2(h);
+                    *reinterpret_cast<uint32_t *>(w + at + XF_PLANE) = f16x2(l);
+                }
+            }
+        };
+        auto arrive = [&](int k) {  // operands of stage k written, sums of stage k - 2 read
+            tc::fence_proxy_async();
+            tc::fence_before_sync();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(tc::smem_u32(&bars[k & 1]));
+        };
+        // this thread's sums: row (warp & 3) * 32 + lane, columns col0 .. col0 + nb / 2, of
+        // the channel slot that the row belongs to
+        const int quarter = warp & 3, cg = warp >> 2;
+        const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
+        const int slot = quarter * 32 / SLOT, q_el = (cg & 1) * (nb / 2);
+        const int col0 = slot * SLOT + (cg >> 1) * nb + q_el;
+        int r_el = quarter * 32 + lane - slot * SLOT;  // element of the row
+        r_el = r_el >= nb ? r_el - nb : r_el;
+        r_el = min(r_el, EB - 1);
+        constexpr int NC = EB / 4;  // pairs of columns
+        float2 acc[NC];
+#pragma unroll
+        for (int i = 0; i < NC; i++) acc[i] = make_float2(0.f, 0.f);
+        // second-level sums, after the operands: each thread its own entries until the end
+        float *D = reinterpret_cast<float *>(smem + 2 * STAGE);
+        float *drow = D + (quarter * 32 + lane) * XF_DS + col0;
+        auto flush = [&](bool first) {
+#pragma unroll
+            for (int j = 0; j < NC; j++)
+                if (2 * j < nb / 2) {
+                    drow[2 * j] = first ? acc[j].x : drow[2 * j] + acc[j].x;
+                    drow[2 * j + 1] = first ? acc[j].y : drow[2 * j + 1] + acc[j].y;
+                    acc[j] = make_float2(0.f, 0.f);
+                }
+        };
+        auto drain = [&](int k) {
+            const uint32_t d = tmem + (uint32_t)((k & 1) * 256) + lane_off + (uint32_t)col0;
+            const float sr = s_inv[k & 3][0][slot * EB + r_el];
+            const float2 sr2 = make_float2(sr, sr);
+            const float *sq = &s_inv[k & 3][sep ? 1 : 0][slot * EB + q_el];
+#pragma unroll
+            for (int c = 0; c < 2 * NC; c += 8) {
+                if (c >= nb / 2) break;  // uniform
+                uint32_t v[8], w[8];
+                tc::tmem_ld8(d + c, v);
+                tc::tmem_ld8(d + 128 + c, w);
+                tc::tmem_ld_wait();
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const float2 t = __fadd2_rn(
+                        make_float2(__uint_as_float(v[2 * j]), __uint_as_float(v[2 * j + 1])),
+                        make_float2(__uint_as_float(w[2 * j]), __uint_as_float(w[2 * j + 1])));
+                    const float2 f = __fmul2_rn(sr2, *reinterpret_cast<const float2 *>(sq + c + 2 * j));
+                    acc[c / 2 + j] = __ffma2_rn(t, f, acc[c / 2 + j]);
+                }
+            }
+        };
+        bool ok = true;
+        for (int k = 0; k < min(2, nstage); k++) {
+            load(xa, liveA, k);
+            convert(k, 0, liveA);
+            if (sep) {
+                load(xb, liveB, k);
+                convert(k, 1, liveB);
+            }
+            arrive(k);
+        }
+        if (nstage > 2) load(xa, liveA, 2);
+        for (int k = 0; k < nstage; k++) {
+            const int s = k & 1;
+            // the products are complete; all warps' scales of the stage are written
+            ok = ok && tc::mbar_wait(tc::smem_u32(&bars[2 + s]), (k >> 1) & 1) &&
+                 tc::mbar_wait(tc::smem_u32(&bars[s]), (k >> 1) & 1);
+            ok = __all_sync(0xffffffffu, ok);
+            if (!ok) break;
+            tc::fence_after_sync();
+            const bool more = k + 2 < nstage;
+            drain(k);
+            if (more) {
+                convert(k + 2, 0, liveA);
+                if (sep) load(xb, liveB, k + 2);
+            }
+            if (k % XF_FLUSH == XF_FLUSH - 1) flush(k < XF_FLUSH);
+            if (more) {
+                if (sep) convert(k + 2, 1, liveB);
+                arrive(k + 2);
+                if (k + 3 < nstage) load(xa, liveA, k + 3);
+            }
+        }
+        if (!ok && lane == 0) atomicExch(&s_fail, 1);
+        tc::fence_before_sync();
+        flush(nstage < XF_FLUSH);
+        tc::named_barrier(1, 32 * XF_WARPS);
+        const bool fail = s_fail != 0;
+        // alpha v + beta V
+        auto put = [&](float2 *Vc, long at, float2 v) {
+            float2 o = make_float2(a.alpha.x * v.x - a.alpha.y * v.y, a.alpha.x * v.y + a.alpha.y * v.x);
+            if (!a.beta_zero) {
+                const float2 w = Vc[at];
+                o.x += a.beta.x * w.x - a.beta.y * w.y;
+                o.y += a.beta.x * w.y + a.beta.y * w.x;
+            }
+            Vc[at] = o;
+        };
+        for (int sl = 0; sl < NSLOT; sl++) {
+            const long c = ch0 + sl;
+            if (c >= a.nbatch) break;
+            const float2 *Xs = a.Xptrs ? a.Xptrs[c] : a.X + c * a.xstride;
+            float2 *Vc = a.Vptrs ? a.Vptrs[c] : a.V + c * a.vstride;
+            const float *Ds = D + sl * SLOT * XF_DS + sl * SLOT;
+            auto at = [&](int r, int q) { return Ds[r * XF_DS + q]; };
+            // sum over the spectra for row r, column q of the tile (r >= q on the diagonal)
+            auto product = [&](int r, int q) {
+                float2 v = make_float2(at(r, q) + at(nb + r, nb + q), at(nb + r, q) - at(r, nb + q));
+                if (fail || !isfinite(v.x) || !isfinite(v.y))
+                    v = direct_product<BLOCKED>(Xs, a.ld, a.nsp, r0 + r, q0 + q);
+                return v;
+            };
+            if (!sep) {  // the tile's square, the upper half as conjugates
+                for (int i = tid; i < nr * nr; i += 32 * XF_WARPS) {
+                    const int q = i / nr, r = i - q * nr;
+                    float2 v = product(max(r, q), min(r, q));
+                    if (r == q) v.y = 0.f;  // autocorrelations are real
+                    if (r < q) v.y = -v.y;
+                    put(Vc, (long)(q0 + q) * a.ldv + r0 + r, v);
+                }
+            } else {
+                for (int i = tid; i < nr * 64; i += 32 * XF_WARPS) {
+                    const int q = i / nr, r = i - q * nr;
+                    put(Vc, (long)(q0 + q) * a.ldv + r0 + r, product(r, q));
+                }
+                for (int i = tid; i < nr * 64; i += 32 * XF_WARPS) {
+                    const int r = i >> 6, q = i & 63;
+                    const float2 v = product(r, q);
+                    put(Vc, (long)(r0 + r) * a.ldv + q0 + q, make_float2(v.x, -v.y));
+                }
+            }
+        }
+    }
+    __syncthreads();
+    if (warp == XF_WARPS) {
+        tc::fence_after_sync();
+        tc::tmem_dealloc(tmem, 512);
+    }
+}
+
+mdt_status xengine_herm_f32(int ne, long nbatch, int nsp, const float2 *X,
+                            const float2 *const *Xptrs, long ld, long xstride, float2 *V,
+                            float2 *const *Vptrs, long ldv, long vstride, float2 alpha,
+                            float2 beta, bool beta_zero, cudaStream_t stream, int blocked)
+{
+    if (ne <= 0 || nbatch <= 0) return MDT_SUCCESS;
+    // blocked: complex64 between 8-sample blocks; read as 16-byte vectors
+    if (blocked && ld == 0) ld = (long)ne * 8;
+    const bool vectors = !blocked || (((uintptr_t)X & 15) == 0 && !Xptrs && ld % 2 == 0 && xstride % 2 == 0);
+    if (nsp < XF_MIN_SPECTRA || !vectors || ne > (1 << 20))
+        return xengine_simt_f32(ne, nbatch, nsp, X, Xptrs, ld, xstride, V, Vptrs, ldv, vstride, alpha,
+                                beta, beta_zero, stream, blocked);
+    XfArgs a;
+    a.ne = ne;
+    a.nsp = nsp;
+    a.npairs = (int)(cdiv(ne, 64) * (cdiv(ne, 64) + 1) / 2);
+    a.nb = (ne + 7) / 8 * 8;
+    a.X = X;
+    a.Xptrs = Xptrs;
+    a.ld = ld;
+    a.xstride = xstride;
+    a.V = V;
+    a.Vptrs = Vptrs;
+    a.ldv = ldv;
+    a.vstride = vstride;
+    a.alpha = alpha;
+    a.beta = beta;
+    a.beta_zero = beta_zero ? 1 : 0;
+    a.nbatch = nbatch;
+    auto launch = [&](auto kern, bool off, long blocks) -> mdt_status {
+        if (blocks > 0x7fffffffL) return invalid("xengine: grid too large");
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)xf_smem(off));
+        if (e != cudaSuccess) return cuda_status(e, "xengine smem attribute");
+        kern<<<(unsigned)blocks, XF_THREADS, xf_smem(off), stream>>>(a);
+        return launch_status("xengine_f32_kernel");
+    };
+    if (ne > 64)
+        return blocked ? launch(xengine_f32_kernel<true, 128, true>, true, nbatch * a.npairs)
+                       : launch(xengine_f32_kernel<true, 128, false>, true, nbatch * a.npairs);
+    if (ne > 32)
+        return blocked ? launch(xengine_f32_kernel<false, 128, true>, false, nbatch)
+                       : launch(xengine_f32_kernel<false, 128, false>, false, nbatch);
+    if (ne > 16)
+        return blocked ? launch(xengine_f32_kernel<false, 64, true>, false, cdiv(nbatch, 2))
+                       : launch(xengine_f32_kernel<false, 64, false>, false, cdiv(nbatch, 2));
+    return blocked ? launch(xengine_f32_kernel<false, 32, true>, false, cdiv(nbatch, 4))
+                   : launch(xengine_f32_kernel<false, 32, false>, false, cdiv(nbatch, 4));
+}
+
+}  // namespace mdt

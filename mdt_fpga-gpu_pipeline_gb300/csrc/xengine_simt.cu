@@ -1,4 +1,5 @@
-// xengine_simt.cu -- FP32 (SIMT) X-engine: per channel c the Hermitian
+// xengine_simt.cu -- FP32 (SIMT) X-engine, for integrations of fewer spectra
+// than the tensor-core form takes (xengine_f32.cu): per channel c the Hermitian
 // product V_c = alpha * X_c X_c^H (+ beta V_c), computed on the lower
 // triangle only and mirrored, which is the reference's cublasCgemmBatched
 // call (OP_N, OP_C, A == B, alpha = 1/Nspectra, beta = 0;
@@ -20,7 +21,7 @@
 #include <algorithm>
 #include <new>
 
-#include "mdt_common.cuh"
+#include "xengine_f32.cuh"
 
 namespace mdt {
 
@@ -313,7 +314,7 @@ __global__ void __launch_bounds__(XS_THREADS, 3) xengine_herm_f32_kernel(XengArg
     }
 }
 
-mdt_status xengine_herm_f32(int ne, long nbatch, int nsp, const float2 *X,
+mdt_status xengine_simt_f32(int ne, long nbatch, int nsp, const float2 *X,
                             const float2 *const *Xptrs, long ld, long xstride, float2 *V,
                             float2 *const *Vptrs, long ldv, long vstride, float2 alpha,
                             float2 beta, bool beta_zero, cudaStream_t stream, int blocked)
