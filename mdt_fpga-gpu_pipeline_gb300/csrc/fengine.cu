@@ -160,6 +160,11 @@ __global__ void __launch_bounds__(FengCfg<N>::THREADS, FengCfg<N>::MINB) fengine
 
 constexpr int SB8 = 8;  // spectra per block
 
+// Channels from which the spectrum-block kernels run as persistent blocks.
+#ifndef MDT_FENG_PERSIST
+#define MDT_FENG_PERSIST 512
+#endif
+
 // Tap sums of the spectrum-block kernels convert int8 samples with integer
 // and FP32 add instructions instead of the int-to-float conversion unit.
 #ifndef MDT_FENG_I2F_MAGIC
@@ -363,6 +368,7 @@ __device__ __forceinline__ void pfb_block8_to_smem(const FengArgs &a, int s0, in
 // Block decode: blk = (kc * NE + e) * 4 + jsub, s0 = 32 kc + 8 jsub.
 struct Block8 {
     int jsub, e, kc, s0;
+    __device__ __forceinline__ Block8() {}
     __device__ __forceinline__ Block8(int ne, int blk)
     {
         jsub = blk & 3;
@@ -419,6 +425,87 @@ __device__ __forceinline__ void store_c64b(const float2 *fsm, const Block8 &b, f
     }
 }
 
+// Transforms the units u, u + step, ... below nunits, one after the other.
+// unit(u, a, b) gives a unit's arguments and block; next(u) skips units without
+// work; store(a, b) writes the transformed rows.  A unit's input rows are staged
+// while the previous unit's FFT and stores run: the staging buffer is free once the
+// tap sum has read it, so the next unit's copies are issued right after the
+// tap-sum barrier.  The compact twiddle table is filled once.
+template <int N, int NT, class Unit, class Next, class Store>
+__device__ __forceinline__ void fengine_units(int u, int step, int nunits, const float2 *tw, float2 *fsm,
+                                              Unit &&unit, Next &&next, Store &&store)
+{
+    using C = FengBCfg<N>;
+    uint8_t *stage = reinterpret_cast<uint8_t *>(fsm) + C::STAGE_OFF;
+    float2 *tws = reinterpret_cast<float2 *>(reinterpret_cast<uint8_t *>(fsm) + C::TW_OFF);
+    u = next(u);
+    if (u >= nunits) return;
+    {
+        FengArgs a;
+        Block8 b;
+        unit(u, a, b);
+        stage_rows_async<N, NT, C::THREADS>(a, b.s0, b.e, stage);
+    }
+    fft::fill_tw_compact<N>(tws, tw, (int)threadIdx.x, C::THREADS);
+    const int lrow = threadIdx.x / C::TPR;
+    const int t = threadIdx.x - lrow * C::TPR;
+    auto none_load = [](int) { return make_float2(0.f, 0.f); };
+    auto none_store = [](int, float2) {};
+    while (true) {
+        {
+            FengArgs a;
+            Block8 b;
+            unit(u, a, b);
+            // waits for the staged rows; its barrier also orders the previous
+            // unit's stores (reads of the rows) before the new tap sums
+            tapsum_from_stage<N, NT, C::THREADS>(a, b.s0, fsm, C::RSTRIDE, stage);
+        }
+        __syncthreads();  // rows complete, staging buffer free
+        const int un = next(u + step);
+        if (un < nunits) {
+            FengArgs a;
+            Block8 b;
+            unit(un, a, b);
+            stage_rows_async<N, NT, C::THREADS>(a, b.s0, b.e, stage);
+        }
+        fft::transform_row_tws<N, C::TPR, false, false>(fsm + (size_t)lrow * C::RSTRIDE, t, tws, none_load,
+                                                        none_store);
+        FengArgs a;
+        Block8 b;
+        unit(u, a, b);
+        store(a, b, u);
+        if (un >= nunits) break;
+        u = un;
+    }
+}
+
+// Nch >= 512 with NT = 4 or 8: persistent blocks (as many as fit on the GPU at
+// once), each looping over units u = blockIdx.x, blockIdx.x + gridDim.x, ...
+// bf16 F-engine, NE=40, Nch=2048, 8 taps, Nsp=4096: 1.71 ms, a block per unit
+// 2.00; batched f16 F-engine, Nch 2048, 4 taps 2.37 (2.79), Nch 512, 8 taps 2.32
+// (2.37) ms for the jobs of one batch.
+// Otherwise one block per unit (smaller blocks share an SM several at a time;
+// NT = 0, other tap counts, forms the tap sums from global memory).
+template <int N, int NT>
+constexpr bool feng_persistent()
+{
+    return NT > 0 && N >= MDT_FENG_PERSIST;
+}
+
+// Blocks of a spectrum-block launch over `units`.
+template <int N, int NT, class K>
+static cudaError_t feng_grid(K kern, long units, long *grid)
+{
+    using C = FengBCfg<N>;
+    *grid = units;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
+    if (e != cudaSuccess || !feng_persistent<N, NT>()) return e;
+    int per_sm = 0;  // the blocks that fit on the GPU at once
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, C::THREADS, C::SMEM);
+    *grid = std::min(units, (long)std::max(per_sm, 1) * sm_count());
+    return e;
+}
+
 // Work unit u decodes as blockIdx.x does in Block8; units whose 8-spectrum
 // block lies past the last one (the tail of the last 32-spectrum chunk) hold
 // no work.
@@ -428,63 +515,26 @@ __device__ __forceinline__ int next_c64b_unit(int u, int step, int nunits, int n
     return u;
 }
 
-// Nch >= 1024 with NT = 4 or 8: persistent blocks (as many as fit on the GPU at once), each
-// looping over units u = blockIdx.x, blockIdx.x + gridDim.x, ...  A unit's
-// input rows are staged while the previous unit's FFT and stores run: the
-// staging buffer is free once the tap sum has read it, so the next unit's
-// copies are issued right after the tap-sum barrier.  The compact twiddle
-// table is filled once per block.
-// Otherwise one block per unit (smaller blocks already share an SM several
-// at a time; NT = 0, other tap counts, forms the tap sums from global memory).
-template <int N, int NT>
-constexpr bool c64b_persistent()
-{
-    return NT > 0 && N >= 1024;
-}
-
 template <int N, int NT>
 __global__ void __launch_bounds__(FengBCfg<N>::THREADS, FengBCfg<N>::MINB)
     fengine_c64b_kernel(FengArgs a, float2 *__restrict__ XB, int nsb, int nunits)
 {
-    using C = FengBCfg<N>;
     extern __shared__ float2 fsm[];
-    if constexpr (!c64b_persistent<N, NT>()) {
+    if constexpr (!feng_persistent<N, NT>()) {
         const Block8 b(a.ne);
         if (b.kc * 4 + b.jsub >= nsb) return;
         fengine_block8<N, NT>(a, b, fsm);
         store_c64b<N>(fsm, b, XB, a.ne, nsb);
     } else {
-        uint8_t *stage = reinterpret_cast<uint8_t *>(fsm) + C::STAGE_OFF;
-        float2 *tws = reinterpret_cast<float2 *>(reinterpret_cast<uint8_t *>(fsm) + C::TW_OFF);
         const int step = (int)gridDim.x;
-        int u = next_c64b_unit((int)blockIdx.x, step, nunits, a.ne, nsb);
-        if (u >= nunits) return;
-        {
-            const Block8 b(a.ne, u);
-            stage_rows_async<N, NT, C::THREADS>(a, b.s0, b.e, stage);
-        }
-        fft::fill_tw_compact<N>(tws, a.tw, (int)threadIdx.x, C::THREADS);
-        const int lrow = threadIdx.x / C::TPR;
-        const int t = threadIdx.x - lrow * C::TPR;
-        auto none_load = [](int) { return make_float2(0.f, 0.f); };
-        auto none_store = [](int, float2) {};
-        while (true) {
-            const Block8 b(a.ne, u);
-            // waits for the staged rows; its barrier also orders the previous
-            // unit's stores (reads of the rows) before the new tap sums
-            tapsum_from_stage<N, NT, C::THREADS>(a, b.s0, fsm, C::RSTRIDE, stage);
-            __syncthreads();  // rows complete, staging buffer free
-            const int un = next_c64b_unit(u + step, step, nunits, a.ne, nsb);
-            if (un < nunits) {
-                const Block8 bn(a.ne, un);
-                stage_rows_async<N, NT, C::THREADS>(a, bn.s0, bn.e, stage);
-            }
-            fft::transform_row_tws<N, C::TPR, false, false>(fsm + (size_t)lrow * C::RSTRIDE, t, tws,
-                                                            none_load, none_store);
-            store_c64b<N>(fsm, b, XB, a.ne, nsb);
-            if (un >= nunits) break;
-            u = un;
-        }
+        fengine_units<N, NT>(
+            (int)blockIdx.x, step, nunits, a.tw, fsm,
+            [&](int u, FengArgs &ua, Block8 &b) {
+                ua = a;
+                b = Block8(a.ne, u);
+            },
+            [&](int u) { return next_c64b_unit(u, step, nunits, a.ne, nsb); },
+            [&](const FengArgs &, const Block8 &b, int) { store_c64b<N>(fsm, b, XB, a.ne, nsb); });
     }
 }
 
@@ -522,17 +572,13 @@ __device__ __forceinline__ float prep(float x, float sc)
     }
 }
 
-template <int N, int NT, typename H, bool QUANT>
-__global__ void __launch_bounds__(FengBCfg<N>::THREADS, FengBCfg<N>::MINB)
-    fengine_x16_kernel(FengArgs a, uint8_t *__restrict__ X16, int nep, int nkc, float scale,
-                       const float *__restrict__ qscales)
+// The block's 8 spectra of each channel into X16[kc][c][e][128 B] (rows of one
+// (chunk, channel) are contiguous).
+template <int N, typename H, bool QUANT>
+__device__ __forceinline__ void store_x16(const float2 *fsm, const Block8 &b, uint8_t *X16, int nep,
+                                          float scale, const float *qscales)
 {
     using C = FengBCfg<N>;
-    extern __shared__ float2 fsm[];
-    const Block8 b(a.ne);
-    fengine_block8<N, NT>(a, b, fsm);
-
-    // X16[kc][c][e][128 B]: rows of one (chunk, channel) are contiguous
     uint8_t *rowbase = X16 + ((size_t)b.kc * N * nep + b.e) * 128;
     const size_t cstride = (size_t)nep * 128;
     const int pre = (b.jsub ^ (b.e & 7)) << 4, pim = ((4 + b.jsub) ^ (b.e & 7)) << 4;
@@ -556,53 +602,71 @@ __global__ void __launch_bounds__(FengBCfg<N>::THREADS, FengBCfg<N>::MINB)
     }
 }
 
+template <int N, int NT, typename H, bool QUANT>
+__global__ void __launch_bounds__(FengBCfg<N>::THREADS, FengBCfg<N>::MINB)
+    fengine_x16_kernel(FengArgs a, uint8_t *__restrict__ X16, int nep, int nunits, float scale,
+                       const float *__restrict__ qscales)
+{
+    extern __shared__ float2 fsm[];
+    if constexpr (!feng_persistent<N, NT>()) {
+        const Block8 b(a.ne);
+        fengine_block8<N, NT>(a, b, fsm);
+        store_x16<N, H, QUANT>(fsm, b, X16, nep, scale, qscales);
+    } else {
+        fengine_units<N, NT>(
+            (int)blockIdx.x, (int)gridDim.x, nunits, a.tw, fsm,
+            [&](int u, FengArgs &ua, Block8 &b) {
+                ua = a;
+                b = Block8(a.ne, u);
+            },
+            [](int u) { return u; },
+            [&](const FengArgs &, const Block8 &b, int) {
+                store_x16<N, H, QUANT>(fsm, b, X16, nep, scale, qscales);
+            });
+    }
+}
+
 // ------------------------------------------------------------------------
 // Batched f16 F-engine: one launch for every job of a batch that shares
-// (Nch, Ntaps).  Job j owns blocks [blk0[j], blk0[j+1]); within a job the
-// blocks decode as in fengine_x16_kernel.
+// (Nch, Ntaps).  Job j owns units [blk0[j], blk0[j+1]); within a job the
+// units decode as in fengine_x16_kernel.
 template <int N, int NT>
 __global__ void __launch_bounds__(FengBCfg<N>::THREADS, FengBCfg<N>::MINB)
-    fengine_x16_batched_kernel(const FJob *__restrict__ jobs, int njobs, const float2 *tw)
+    fengine_x16_batched_kernel(const FJob *__restrict__ jobs, int njobs, int nunits, const float2 *tw)
 {
-    using C = FengBCfg<N>;
     extern __shared__ float2 fsm[];
-    int j = 0;
-    while (j + 1 < njobs && (int)blockIdx.x >= jobs[j + 1].blk0) j++;
-    const FJob jb = jobs[j];
-    FengArgs a;
-    a.hist = nullptr;
-    a.iq = jb.iq;
-    a.nhist = 0;
-    a.ne = jb.ne;
-    a.ntaps = NT;
-    a.nsp = jb.nsp;
-    a.ngroups = 0;
-    a.win = jb.win;
-    a.tw = tw;
-    a.X = nullptr;
-    const Block8 b(jb.ne, (int)blockIdx.x - jb.blk0);
-    fengine_block8<N, NT>(a, b, fsm);
-
-    uint8_t *rowbase = jb.X16 + ((size_t)b.kc * N * jb.nep + b.e) * 128;
-    const size_t cstride = (size_t)jb.nep * 128;
-    const int pre = (b.jsub ^ (b.e & 7)) << 4, pim = ((4 + b.jsub) ^ (b.e & 7)) << 4;
-    const float sc = jb.scale;
-    for (int c = threadIdx.x; c < N; c += C::THREADS) {
-        float2 v[8];
-#pragma unroll
-        for (int r = 0; r < 8; r++) v[r] = fsm[(size_t)r * C::RSTRIDE + fft::pad(c)];
-        uint4 ure, uim;
-        ure.x = pack2<__half>(v[0].x * sc, v[1].x * sc);
-        ure.y = pack2<__half>(v[2].x * sc, v[3].x * sc);
-        ure.z = pack2<__half>(v[4].x * sc, v[5].x * sc);
-        ure.w = pack2<__half>(v[6].x * sc, v[7].x * sc);
-        uim.x = pack2<__half>(v[0].y * sc, v[1].y * sc);
-        uim.y = pack2<__half>(v[2].y * sc, v[3].y * sc);
-        uim.z = pack2<__half>(v[4].y * sc, v[5].y * sc);
-        uim.w = pack2<__half>(v[6].y * sc, v[7].y * sc);
-        uint8_t *row = rowbase + (size_t)c * cstride;
-        *reinterpret_cast<uint4 *>(row + pre) = ure;
-        *reinterpret_cast<uint4 *>(row + pim) = uim;
+    auto job_of = [&](int u) {
+        int j = 0;
+        while (j + 1 < njobs && u >= __ldg(&jobs[j + 1].blk0)) j++;
+        return j;
+    };
+    auto unit = [&](int u, FengArgs &a, Block8 &b) {
+        const FJob &jb = jobs[job_of(u)];
+        a.hist = nullptr;
+        a.iq = jb.iq;
+        a.nhist = 0;
+        a.ne = jb.ne;
+        a.ntaps = NT;
+        a.nsp = jb.nsp;
+        a.ngroups = 0;
+        a.win = jb.win;
+        a.tw = tw;
+        a.X = nullptr;
+        b = Block8(jb.ne, u - jb.blk0);
+    };
+    auto store = [&](const FengArgs &, const Block8 &b, int u) {
+        const FJob &jb = jobs[job_of(u)];
+        store_x16<N, __half, false>(fsm, b, jb.X16, jb.nep, jb.scale, nullptr);
+    };
+    if constexpr (!feng_persistent<N, NT>()) {
+        FengArgs a;
+        Block8 b;
+        unit((int)blockIdx.x, a, b);
+        fengine_block8<N, NT>(a, b, fsm);
+        store(a, b, (int)blockIdx.x);
+    } else {
+        fengine_units<N, NT>((int)blockIdx.x, (int)gridDim.x, nunits, tw, fsm, unit,
+                             [](int u) { return u; }, store);
     }
 }
 
@@ -679,13 +743,13 @@ struct Feng16Run {
         mdt_status st;
         a.tw = fft_twiddles(N, &st);
         if (!a.tw) return st;
-        long blocks = (long)a.ne * nkc * 4;
-        if (blocks > 0x7fffffffL) return invalid("fengine_x16: grid too large");
+        const long units = (long)a.ne * nkc * 4;
+        if (units > 0x7fffffffL) return invalid("fengine_x16: grid too large");
         auto kern = qscales ? fengine_x16_kernel<N, NT, H, true> : fengine_x16_kernel<N, NT, H, false>;
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)C::SMEM);
-        if (e != cudaSuccess) return cuda_status(e, "fengine_x16 smem attribute");
-        kern<<<(unsigned)blocks, C::THREADS, C::SMEM, stream>>>(a, X16, nep, nkc, scale, qscales);
+        long grid = 0;
+        cudaError_t e = feng_grid<N, NT>(kern, units, &grid);
+        if (e != cudaSuccess) return cuda_status(e, "fengine_x16 launch shape");
+        kern<<<(unsigned)grid, C::THREADS, C::SMEM, stream>>>(a, X16, nep, (int)units, scale, qscales);
         return launch_status("fengine_x16_kernel");
     }
 };
@@ -707,21 +771,12 @@ struct FengBRun {
         mdt_status st = MDT_SUCCESS;
         a.tw = tw_concat ? tw_concat + (N - 32) : fft_twiddles(N, &st);
         if (!a.tw) return st;
-        cudaError_t e = cudaFuncSetAttribute(fengine_c64b_kernel<N, NT>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)C::SMEM);
-        if (e != cudaSuccess) return cuda_status(e, "fengine_c64b smem attribute");
         const long nkc = (nsb + 3) / 4;
         const long units = (long)a.ne * nkc * 4;
         if (units > 0x7fffffffL) return invalid("fengine_c64b: grid too large");
-        long grid = units;
-        if (c64b_persistent<N, NT>()) {  // the blocks that fit on the GPU at once
-            int per_sm = 0;
-            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fengine_c64b_kernel<N, NT>,
-                                                              C::THREADS, C::SMEM);
-            if (e != cudaSuccess) return cuda_status(e, "fengine_c64b occupancy");
-            grid = std::min(units, (long)std::max(per_sm, 1) * sm_count());
-        }
+        long grid = 0;
+        cudaError_t e = feng_grid<N, NT>(fengine_c64b_kernel<N, NT>, units, &grid);
+        if (e != cudaSuccess) return cuda_status(e, "fengine_c64b launch shape");
         if (grid == 0) return MDT_SUCCESS;
         fengine_c64b_kernel<N, NT><<<(unsigned)grid, C::THREADS, C::SMEM, stream>>>(a, XB, nsb,
                                                                                    (int)units);
@@ -776,13 +831,12 @@ struct FengBatchRun {
             mdt_status st;
             const float2 *tw = fft_twiddles(N, &st);
             if (!tw) return st;
-            cudaError_t e = cudaFuncSetAttribute(fengine_x16_batched_kernel<N, NT>,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 (int)C::SMEM);
-            if (e != cudaSuccess) return cuda_status(e, "batched F-engine smem attribute");
             if (nblocks > 0x7fffffffL) return invalid("batched F-engine: grid too large");
-            fengine_x16_batched_kernel<N, NT><<<(unsigned)nblocks, C::THREADS, C::SMEM, stream>>>(
-                jobs, njobs, tw);
+            long grid = 0;
+            cudaError_t e = feng_grid<N, NT>(fengine_x16_batched_kernel<N, NT>, nblocks, &grid);
+            if (e != cudaSuccess) return cuda_status(e, "batched F-engine launch shape");
+            fengine_x16_batched_kernel<N, NT><<<(unsigned)grid, C::THREADS, C::SMEM, stream>>>(
+                jobs, njobs, (int)nblocks, tw);
             return launch_status("fengine_x16_batched_kernel");
         }
     }
