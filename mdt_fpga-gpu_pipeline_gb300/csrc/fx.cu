@@ -12,16 +12,12 @@
 #include <vector>
 
 #include "fengine.cuh"
-#include "mdt_common.cuh"
+#include "xengine_f32.cuh"
 
 namespace mdt {
 mdt_status check_dims(int ne, int nch, int ntaps, int nsp);
 mdt_status fengine_f32(int ne, int nch, int ntaps, int nsp, const int8_t *hist, int nhist,
                        const int8_t *iq, const float *win, float2 *X, cudaStream_t stream);
-mdt_status xengine_herm_f32(int ne, long nbatch, int nsp, const float2 *X,
-                            const float2 *const *Xptrs, long ld, long xstride, float2 *V,
-                            float2 *const *Vptrs, long ldv, long vstride, float2 alpha,
-                            float2 beta, bool beta_zero, cudaStream_t stream, int blocked);
 mdt_status fengine_c64b(int ne, int nch, int ntaps, int nsp, const int8_t *hist, int nhist,
                         const int8_t *iq, const float *win, float2 *XB, cudaStream_t stream);
 const float2 *fft_twiddles(int n, mdt_status *st);
@@ -147,6 +143,9 @@ mdt_status one_integration(mdt_fx_plan p, const int8_t *hist, int nhist, const i
     if (d.precision == MDT_PREC_FP32) {
         // F-output in the 8-spectrum blocked layout XB (fengine.cuh)
         const long nsb = (d.nspectra + 7) / 8;
+        // An FP64 sum over integrations may be saved and continued later: its terms come
+        // from the one kernel that rounds the same way at every number of spectra.
+        const auto xengine = p->acc ? mdt::xengine_simt_f32 : mdt::xengine_herm_f32;
         if (d.nchannels <= 2048)
             st = mdt::fengine_c64b(d.nelements, d.nchannels, d.ntaps, d.nspectra, hist, nhist, iq,
                                    p->window, p->X, p->stream);
@@ -158,22 +157,22 @@ mdt_status one_integration(mdt_fx_plan p, const int8_t *hist, int nhist, const i
                                   iq, p->window, p->X, p->stream);
             if (st != MDT_SUCCESS) return st;
             if (t1) cudaEventRecord(t1, p->stream);
-            st = mdt::xengine_herm_f32(d.nelements, d.nchannels, d.nspectra, p->X, nullptr,
-                                       d.nelements, (long)d.nspectra * d.nelements,
-                                       (float2 *)vis, nullptr, d.nelements,
-                                       (long)d.nelements * d.nelements,
-                                       make_float2(1.0f / d.nspectra, 0.f), make_float2(0.f, 0.f),
-                                       true, p->stream, 0);
+            st = xengine(d.nelements, d.nchannels, d.nspectra, p->X, nullptr,
+                         d.nelements, (long)d.nspectra * d.nelements,
+                         (float2 *)vis, nullptr, d.nelements,
+                         (long)d.nelements * d.nelements,
+                         make_float2(1.0f / d.nspectra, 0.f), make_float2(0.f, 0.f),
+                         true, p->stream, 0);
         } else {
             if (st != MDT_SUCCESS) return st;
             if (t1) cudaEventRecord(t1, p->stream);
-            st = mdt::xengine_herm_f32(d.nelements, d.nchannels, d.nspectra, p->X, nullptr,
-                                       mdt::xb_block_stride(d.nelements, d.nchannels, nsb),
-                                       mdt::xb_chan_stride(d.nelements, d.nchannels, nsb),
-                                       (float2 *)vis, nullptr,
-                                       d.nelements, (long)d.nelements * d.nelements,
-                                       make_float2(1.0f / d.nspectra, 0.f), make_float2(0.f, 0.f),
-                                       true, p->stream, 1);
+            st = xengine(d.nelements, d.nchannels, d.nspectra, p->X, nullptr,
+                         mdt::xb_block_stride(d.nelements, d.nchannels, nsb),
+                         mdt::xb_chan_stride(d.nelements, d.nchannels, nsb),
+                         (float2 *)vis, nullptr,
+                         d.nelements, (long)d.nelements * d.nelements,
+                         make_float2(1.0f / d.nspectra, 0.f), make_float2(0.f, 0.f),
+                         true, p->stream, 1);
         }
         if (st == MDT_SUCCESS && p->acc) {
             long n = (long)d.nchannels * d.nelements * d.nelements;
