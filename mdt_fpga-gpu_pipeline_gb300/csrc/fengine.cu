@@ -36,11 +36,13 @@ namespace mdt {
 #define MDT_FENG_SM_THREADS 1024
 #endif
 
-// Threads per row: one radix-16 butterfly per thread and pass (at least 4).  With
-// N/8 threads half of them wait out the radix-16 passes, and the tap sum has one
-// channel per thread instead of a packed pair: the batched f16 F-engine of four
-// jobs with Nch 512 (546 M samples, 8 taps) takes 2.37 ms, with N/8 threads 3.63.
-constexpr int feng_tpr(int n) { return n / 16 < 4 ? 4 : n / 16; }
+// Threads per row: from 256 channels on one radix-16 butterfly per thread and pass.
+// With N/8 threads half of them wait out the radix-16 passes, and the tap sum has one
+// channel per thread instead of a packed pair: the batched f16 F-engine of four jobs
+// with Nch 512 (546 M samples, 8 taps) takes 2.37 ms, with N/8 threads 3.63.  Blocks of
+// shorter rows have too few threads for that and take N/8 (400,000 rows of Nch 64, 4
+// taps, FP32: 101 us, with N/16 109; of Nch 128 172 and 182).
+constexpr int feng_tpr(int n) { return n < 256 ? n / 8 : n / 16; }
 
 template <int N>
 struct FengCfg {
