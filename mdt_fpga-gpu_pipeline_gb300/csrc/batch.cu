@@ -137,12 +137,19 @@ std::vector<mdt::XWork> build_work(mdt_fx_batch b, TuneChoice c)
     std::vector<mdt::XWork> work;
     std::vector<long> cost;
     mdt::TcTile tiles[160];
+    long entries = 0;
+    for (int j = 0; j < b->njobs; j++)
+        entries += (long)b->d[j].nchannels *
+                   mdt::make_tiles(b->d[j].nelements, b->nep[j], c.maxw, tiles);
     for (int j = 0; j < b->njobs; j++) {
         const mdt_fx_desc &d = b->d[j];
         const int nt = mdt::make_tiles(d.nelements, b->nep[j], c.maxw, tiles);
-        for (int ch = 0; ch < d.nchannels; ch++)
+        // small arrays: the rows of several channels as one tile
+        const int grp = nt == 1 ? mdt::tc_group(b->nep[j], entries, 2) : 1;
+        for (int ch = 0; ch < d.nchannels; ch += grp)
             for (int t = 0; t < nt; t++) {
-                work.push_back({j, ch, tiles[t]});
+                if (grp > 1) tiles[t].n = (int16_t)(b->nep[j] * std::min(grp, d.nchannels - ch));
+                work.push_back({j, ch, grp > 1 ? 1 : 0, tiles[t]});
                 cost.push_back((long)b->nkc[j] * (tiles[t].n + (tiles[t].a_sep ? 128 : 0)));
             }
     }

@@ -21,6 +21,10 @@
 // imaginary part is antisymmetric: Im V = G - G^T with G = X_im X_re^T, so
 // only G += A2 B0 + A3 B1 is accumulated (six MMAs instead of eight) and the
 // epilogue forms G[r][q] - G[q][r] through shared memory.
+// An MMA of this shape takes the tensor core some 110 cycles however few columns
+// it has, so arrays of up to 64 (32, 16) padded rows take two (four, eight)
+// channels at once: their rows are consecutive in the operand, and the products
+// between channels are not read.
 // A block owns one (channel, row tile of 128 elements, column chunk of up to
 // 256 elements) of the lower triangle: only tiles on or below the diagonal
 // are computed; the epilogue writes the lower triangle and its conjugate
@@ -94,6 +98,7 @@ struct TcArgs {
     long chunk_bytes;   // stride between 32-spectrum chunks: Nch * NEp * 128
     long chan_bytes;    // stride between channels: NEp * 128
     int ne, nep, nkc;
+    int nch, group;     // channels, and channels of a block (see tc_group)
     int ntiles;
     int ab_fmt;         // 0 = f16, 1 = bf16
     float alpha;        // applied to the accumulators (1/(Nsp * scale^2))
@@ -110,7 +115,8 @@ constexpr int TC_WIN = 16;  // K-chunks (of 32 spectra) per exact accumulation w
 // STAGES-deep ring of (B: BROWS rows, A: 128 rows) stages; BROWS 256 with 4
 // stages (one block per SM) or 128 with 3 stages (two blocks per SM, so one
 // block's epilogue overlaps the other's products).
-template <int KIND, int BROWS, int STAGES>  // KIND 0: f16 / bf16, float results; 1: exact int8
+// KIND 0: f16 / bf16, float results; 1: exact int8.  GROUPS: blocks may take several channels
+template <int KIND, int BROWS, int STAGES, bool GROUPS>
 __global__ void __launch_bounds__(tc_threads(KIND), (KIND == 0 && BROWS == 128 ? 2 : 1))
     xengine_tc_kernel(const __grid_constant__ TcArgs a)
 {
@@ -127,9 +133,12 @@ __global__ void __launch_bounds__(tc_threads(KIND), (KIND == 0 && BROWS == 128 ?
     uint32_t *tmem_slot = (uint32_t *)(bars + 2 * STAGES + 5);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int ch = blockIdx.x / a.ntiles;
-    const TcTile tile = a.tiles[blockIdx.x - ch * a.ntiles];
-    const int N = tile.n;
+    const int blk = blockIdx.x / a.ntiles;
+    const TcTile tile = a.tiles[blockIdx.x - blk * a.ntiles];
+    // a group of channels is one tile of their rows, one after the other
+    const int ch = GROUPS ? blk * a.group : blk;
+    const int ngrp = GROUPS ? min(a.group, a.nch - ch) : 1;
+    const int N = tile.n * ngrp;
     // diagonal tile: rows and columns are the same elements (A read from B's rows)
     const bool sym = tc_sym(KIND, BROWS) && tile.r0 == tile.q0 && !tile.a_sep;
     constexpr int NCOLMUL = (KIND == 0) ? 2 : 4;  // TMEM columns per output column
@@ -233,14 +242,13 @@ __global__ void __launch_bounds__(tc_threads(KIND), (KIND == 0 && BROWS == 128 ?
         // lane quarter w % 4, columns [32 cg, 32 cg + 32) with cg = (w - 2) / 4, and
         // keeps the int32 running sums of its row and 32 columns in registers
         const int quarter = warp & 3, cg = (warp - 2) >> 2;
-        const int r = tile.r0 + quarter * 32 + lane;
         const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
         const int nwin = (a.nkc + TC_WIN - 1) / TC_WIN;
+        const int r = tile.r0 + quarter * 32 + lane;
         float2 *Vc = a.V ? a.V + (long)ch * a.ne * a.ne : nullptr;
         double2 *Ac = a.Vacc ? a.Vacc + (long)ch * a.ne * a.ne : nullptr;
         int2 *Rc = a.raw ? a.raw + (long)ch * a.ne * a.ne : nullptr;
-        const float qs = __ldg(a.qscales + ch);
-        const float alpha = a.alpha / (qs * qs);
+        const float qs = __ldg(a.qscales + ch), alpha = a.alpha / (qs * qs);
         int rr[32], ri[32];
 #pragma unroll
         for (int j = 0; j < 32; j++) rr[j] = ri[j] = 0;
@@ -268,30 +276,52 @@ __global__ void __launch_bounds__(tc_threads(KIND), (KIND == 0 && BROWS == 128 ?
             __syncwarp();
             if (lane == 0) tc::mbar_arrive(tc::smem_u32(&win_empty[h]));
         }
-        if (ok && r < a.ne) {
+        auto store = [&](int j, int q, int r, float2 *Vc, double2 *Ac, int2 *Rc, float alpha) {
+            const int ire = rr[j];
+            const int iim = (q == r) ? 0 : ri[j];
+            const long lo = (long)q * a.ne + r, up = (long)r * a.ne + q;
+            if (Rc) {
+                Rc[lo] = make_int2(ire, iim);
+                if (q != r) Rc[up] = make_int2(ire, -iim);
+            }
+            const float re = (float)ire * alpha, im = (float)iim * alpha;
+            if (Vc) {
+                Vc[lo] = make_float2(re, im);
+                if (q != r) Vc[up] = make_float2(re, -im);
+            }
+            if (Ac) {
+                double2 x = Ac[lo];
+                Ac[lo] = make_double2(x.x + (double)re, x.y + (double)im);
+                if (q != r) {
+                    double2 y = Ac[up];
+                    Ac[up] = make_double2(y.x + (double)re, y.y - (double)im);
+                }
+            }
+        };
+        if constexpr (!GROUPS) {
+            if (ok && r < a.ne) {
 #pragma unroll
-            for (int j = 0; j < 32; j++) {
-                const int q = tile.q0 + 32 * cg + j;
-                if (32 * cg + j >= N || q >= a.ne || q > r) continue;
-                const int ire = rr[j];
-                const int iim = (q == r) ? 0 : ri[j];
-                const long lo = (long)q * a.ne + r, up = (long)r * a.ne + q;
-                if (Rc) {
-                    Rc[lo] = make_int2(ire, iim);
-                    if (q != r) Rc[up] = make_int2(ire, -iim);
+                for (int j = 0; j < 32; j++) {
+                    const int q = tile.q0 + 32 * cg + j;
+                    if (32 * cg + j >= N || q >= a.ne || q > r) continue;
+                    store(j, q, r, Vc, Ac, Rc, alpha);
                 }
-                const float re = (float)ire * alpha, im = (float)iim * alpha;
-                if (Vc) {
-                    Vc[lo] = make_float2(re, im);
-                    if (q != r) Vc[up] = make_float2(re, -im);
-                }
-                if (Ac) {
-                    double2 x = Ac[lo];
-                    Ac[lo] = make_double2(x.x + (double)re, x.y + (double)im);
-                    if (q != r) {
-                        double2 y = Ac[up];
-                        Ac[up] = make_double2(y.x + (double)re, y.y - (double)im);
-                    }
+            }
+        } else {
+#pragma unroll
+            for (int hf = 0; hf < 2; hf++) {
+                // the channel of these 16 columns: rows of its other channels are skipped
+                const int n0 = 32 * cg + 16 * hf, cc = n0 / tile.n, skip = cc * tile.n;
+                const int rc = r - skip;
+                if (!ok || n0 >= N || rc < 0 || rc >= a.ne) continue;
+                const long vo = (long)cc * a.ne * a.ne;
+                const float qc = __ldg(a.qscales + ch + cc);
+#pragma unroll
+                for (int j = 0; j < 16; j++) {
+                    const int q = tile.q0 + n0 - skip + j;
+                    if (q >= a.ne || q > rc) continue;
+                    store(16 * hf + j, q, rc, Vc ? Vc + vo : nullptr, Ac ? Ac + vo : nullptr,
+                          Rc ? Rc + vo : nullptr, a.alpha / (qc * qc));
                 }
             }
         }
@@ -302,8 +332,8 @@ __global__ void __launch_bounds__(tc_threads(KIND), (KIND == 0 && BROWS == 128 ?
         ok = tc::mbar_wait_sleep(tc::smem_u32(&bars[2 * STAGES]), 0);
         tc::fence_after_sync();
         const int quarter = warp & 3, half = (warp - 2) >> 2;
-        const int r = tile.r0 + quarter * 32 + lane;
         const uint32_t lane_off = (uint32_t)(quarter * 32) << 16;
+        int r = tile.r0 + quarter * 32 + lane, rbase = tile.r0 + quarter * 32, qb = tile.q0;
         float2 *Vc = a.V ? a.V + (long)ch * a.ne * a.ne : nullptr;
         double2 *Ac = a.Vacc ? a.Vacc + (long)ch * a.ne * a.ne : nullptr;
         // this warp's columns [c0, c1): N is a multiple of 16, halves are too
@@ -314,7 +344,6 @@ __global__ void __launch_bounds__(tc_threads(KIND), (KIND == 0 && BROWS == 128 ?
         // stage ring is idle once every MMA has completed) in 16-column blocks
         // so that it is written along q as well, two rows per store.
         float2 *tb = reinterpret_cast<float2 *>(smem) + (size_t)(warp - 2) * 16 * 33;  // [q][r]
-        const int rbase = tile.r0 + quarter * 32;
         // diagonal tile: G (the Im accumulator) row by row into shared memory, so
         // that each thread can read the transposed entry G[q][r] (tile-local)
         float *gs = reinterpret_cast<float *>(smem + TC_TB_BYTES);
@@ -330,13 +359,25 @@ __global__ void __launch_bounds__(tc_threads(KIND), (KIND == 0 && BROWS == 128 ?
         }
         if (tc_sym(KIND, BROWS)) tc::named_barrier(1, 256);  // the eight epilogue warps
         for (int n0 = c0; n0 < c1; n0 += 16) {
+            if constexpr (GROUPS) {
+                // the channel of these 16 columns (tile.n is a multiple of 16): rows of other
+                // channels of the group are skipped
+                const int cc = n0 / tile.n, skip = cc * tile.n;
+                rbase = tile.r0 + quarter * 32 - skip;  // the warp's first row in it
+                if (rbase + 32 <= 0 || rbase >= tile.n) continue;
+                r = rbase + lane;
+                qb = tile.q0 - skip;
+                const long vo = (long)(ch + cc) * a.ne * a.ne;
+                Vc = a.V ? a.V + vo : nullptr;
+                Ac = a.Vacc ? a.Vacc + vo : nullptr;
+            }
             uint32_t vr[16], vi[16];
             tc::tmem_ld16(d_re + lane_off + n0, vr);
             tc::tmem_ld16(d_im + lane_off + n0, vi);
             tc::tmem_ld_wait();
 #pragma unroll
             for (int j = 0; j < 16; j++) {
-                const int q = tile.q0 + n0 + j;
+                const int q = qb + n0 + j;
                 const bool live = ok && r < a.ne && q < a.ne && q <= r;
                 const float re = live ? __uint_as_float(vr[j]) * a.alpha : 0.0f;
                 const float g = sym && live ? gs[(n0 + j) * TC_GS + rl] : 0.0f;
@@ -351,8 +392,8 @@ __global__ void __launch_bounds__(tc_threads(KIND), (KIND == 0 && BROWS == 128 ?
                 }
             }
             __syncwarp();
-            // mirror: rows rbase + rr (two per step), columns q = tile.q0 + n0 + (lane & 15)
-            const int qc = lane & 15, q = tile.q0 + n0 + qc;
+            // mirror: rows rbase + rr (two per step), columns q = qb + n0 + (lane & 15)
+            const int qc = lane & 15, q = qb + n0 + qc;
 #pragma unroll 4
             for (int i = 0; i < 16; i++) {
                 const int rr = 2 * i + (lane >> 4), rm = rbase + rr;
@@ -503,7 +544,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
             tc::fence_after_sync();
             const uint32_t d_re = tmem + (uint32_t)(h * 256), d_im = d_re + (uint32_t)N;
             const int rl = quarter * 32 + lane;
-            const int r = wk.tile.r0 + rl;
+            // columns of a channel: all of the entry's, or a group's rows one after the other
+            const int cw = wk.grouped ? jb.nep : N;
             if (sym) {  // G row by row into shared memory, for the transposed entries
                 for (int n0 = 0; n0 < N; n0 += 16) {
                     uint32_t vg[16];
@@ -515,9 +557,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                 }
                 tc::named_barrier(1, 128);
             }
-            // no visibility buffer (autotuning before the first execute): no writes
-            float2 *Vc = jb.V ? jb.V + (long)wk.ch * jb.ne * jb.ne : nullptr;
             for (int n0 = 0; n0 < N; n0 += 16) {
+                const int cc = n0 / cw, skip = cc * cw;
+                const int rw = wk.tile.r0 + quarter * 32 - skip;  // the warp's first row in it
+                if (wk.grouped && (rw + 32 <= 0 || rw >= cw)) continue;
+                const int r = rw + lane, qb = wk.tile.q0 + n0 - skip;
+                // no visibility buffer (autotuning before the first execute): no writes
+                float2 *Vc = jb.V ? jb.V + (long)(wk.ch + cc) * jb.ne * jb.ne : nullptr;
                 uint32_t vr[16], vi[16];
                 tc::tmem_ld16(d_re + lane_off + n0, vr);
                 tc::tmem_ld16(d_im + lane_off + n0, vi);
@@ -525,7 +571,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                 if (!ok || r >= jb.ne || !Vc) continue;
 #pragma unroll
                 for (int j = 0; j < 16; j++) {
-                    const int q = wk.tile.q0 + n0 + j;
+                    const int q = qb + j;
                     if (q >= jb.ne || q > r) continue;
                     const float re = __uint_as_float(vr[j]) * jb.alpha;
                     const float g = sym ? gs[(n0 + j) * TC_GS + rl] : 0.0f;
@@ -591,6 +637,20 @@ int make_tiles(int ne, int nep, int maxw, TcTile *tiles)
     return n;
 }
 
+// Channels that a block takes: as many as 128 rows hold, but no more than leave each
+// SM its per_sm blocks (two; one in the exact int8 mode), since a block's epilogue
+// grows with its channels.  One against
+// two, four and eight channels: NE=10, Nch=2048, Nsp=2048 203, 119, 71 and 48 us;
+// NE=30, Nch=1024, Nsp=512 43, 28 and 18 us; NE=60, Nch=1024, Nsp=2048 148 and 108 us;
+// where too few blocks are left (NE=10, Nch=128, Nsp=128) 6.1, 6.3, 8.1 and 8.6 us.
+int tc_group(int nep, long blocks, int per_sm)
+{
+    const int most = nep <= 16 ? 8 : nep <= 32 ? 4 : nep <= 64 ? 2 : 1;
+    int g = 1;
+    while (g < most && cdiv(blocks, g) > (long)per_sm * sm_count()) g *= 2;
+    return g;
+}
+
 int x16_padded_rows(int ne) { return (ne + 15) / 16 * 16; }
 int x16_chunks(int nsp) { return (nsp + 31) / 32; }
 
@@ -622,8 +682,10 @@ mdt_status xengine_tc(int ne, int nch, int nsp, const void *X16, int ab_fmt, flo
     const int maxw = wide ? 256 : 128;
     a.ntiles = make_tiles(ne, a.nep, maxw, a.tiles);
     if (a.ntiles <= 0) return invalid("xengine_tc: too many tiles");
-    long blocks = (long)nch * a.ntiles;
-    if (blocks > 0x7fffffffL) return invalid("xengine_tc: grid too large");
+    a.nch = nch;
+    a.group = wide ? 1 : tc_group(a.nep, nch, 2);
+    if ((long)nch * a.ntiles > 0x7fffffffL) return invalid("xengine_tc: grid too large");
+    const long blocks = cdiv(nch, a.group) * a.ntiles;
     auto launch = [&](auto kern, size_t smem) -> mdt_status {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)smem);
@@ -631,8 +693,9 @@ mdt_status xengine_tc(int ne, int nch, int nsp, const void *X16, int ab_fmt, flo
         kern<<<(unsigned)blocks, tc_threads(0), smem, stream>>>(a);
         return launch_status("xengine_tc_kernel");
     };
-    return wide ? launch(xengine_tc_kernel<0, 256, 4>, tc_smem(0, 256, 4))
-                : launch(xengine_tc_kernel<0, 128, 3>, tc_smem(0, 128, 3));
+    if (wide) return launch(xengine_tc_kernel<0, 256, 4, false>, tc_smem(0, 256, 4));
+    return a.group > 1 ? launch(xengine_tc_kernel<0, 128, 3, true>, tc_smem(0, 128, 3))
+                       : launch(xengine_tc_kernel<0, 128, 3, false>, tc_smem(0, 128, 3));
 }
 
 // Exact int8 mode: X16 holds integers in [-127, 127] (f16) requantised with
@@ -659,13 +722,15 @@ mdt_status xengine_q8(int ne, int nch, int nsp, const void *X16, const float *qs
     a.raw = raw;
     a.ntiles = make_tiles(ne, a.nep, 128, a.tiles);
     if (a.ntiles <= 0) return invalid("xengine_q8: too many tiles");
-    cudaError_t e = cudaFuncSetAttribute(xengine_tc_kernel<1, 128, 4>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+    a.nch = nch;
+    a.group = tc_group(a.nep, nch, 1);
+    auto kern = a.group > 1 ? xengine_tc_kernel<1, 128, 4, true> : xengine_tc_kernel<1, 128, 4, false>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)tc_smem(1, 128, 4));
     if (e != cudaSuccess) return cuda_status(e, "xengine_q8 smem attribute");
-    long blocks = (long)nch * a.ntiles;
-    if (blocks > 0x7fffffffL) return invalid("xengine_q8: grid too large");
-    xengine_tc_kernel<1, 128, 4><<<(unsigned)blocks, tc_threads(1), tc_smem(1, 128, 4), stream>>>(a);
+    if ((long)nch * a.ntiles > 0x7fffffffL) return invalid("xengine_q8: grid too large");
+    const long blocks = cdiv(nch, a.group) * a.ntiles;
+    kern<<<(unsigned)blocks, tc_threads(1), tc_smem(1, 128, 4), stream>>>(a);
     return launch_status("xengine_tc_kernel<exact int8>");
 }
 

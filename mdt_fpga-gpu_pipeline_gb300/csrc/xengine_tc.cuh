@@ -22,6 +22,7 @@ struct XJob {
 // One work entry of a batched X-engine launch: a tile of one channel of one job.
 struct XWork {
     int job, ch;
+    int grouped;  // the tile holds the rows of several channels from ch on (tc_group)
     TcTile tile;
 };
 
@@ -30,6 +31,9 @@ constexpr int TCB_MAXW = 128;  // widest column chunk of the batched X-engine
 // Lower-triangle tiles (row tiles of 128, column chunks of <= maxw) for NE
 // elements padded to nep rows; returns the count or -1 if more than 160.
 int make_tiles(int ne, int nep, int maxw, TcTile *tiles);
+// Channels whose rows one tile takes together (1, 2, 4 or 8), by the padded rows and
+// the blocks or work entries that there are at one channel each and an SM holds.
+int tc_group(int nep, long blocks, int per_sm);
 int x16_padded_rows(int ne);
 int x16_chunks(int nsp);
 mdt_status xengine_tc_batched(const XJob *jobs, const XWork *work, int nwork, int *err,
