@@ -176,8 +176,8 @@ __global__ void __launch_bounds__(32 * GG_PH, 4)
 // eight independent loads per thread, the element index formed once per
 // thread and row half.  NE=64, Nch=512, Nsp=2048: 210 us (5.1 TB/s), with
 // 32 x 32 tiles and a 64-bit division per value 233 us.
-constexpr int FA_T = 64;
-__global__ void __launch_bounds__(512)
+template <int FA_T>
+__global__ void __launch_bounds__(8 * FA_T)
     fout_adjoint_kernel(int ne, int nch, long rows, const float2 *__restrict__ dY,
                         const float2 *__restrict__ g, float2 *__restrict__ dF)
 {
@@ -185,98 +185,107 @@ __global__ void __launch_bounds__(512)
     const long r0 = (long)blockIdx.x * FA_T;
     const int c0 = blockIdx.y * FA_T, lane = threadIdx.x, warp = threadIdx.y;
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
+    for (int h = 0; h < FA_T / 32; h++) {
         const long r = r0 + 32 * h + lane;
         const int e = (int)(r % ne);
 #pragma unroll
-        for (int y = 0; y < FA_T / 16; y++) {
-            const int c = c0 + warp + 16 * y;
+        for (int y = 0; y < 4; y++) {
+            const int c = c0 + warp + FA_T / 4 * y;
             if (c < nch && r < rows) {
                 const float2 gv = g ? __ldg(g + (long)c * ne + e) : make_float2(1.f, 0.f);
-                t[warp + 16 * y][32 * h + lane] = cmul(cconj(gv), __ldg(dY + (long)c * rows + r));
+                t[warp + FA_T / 4 * y][32 * h + lane] = cmul(cconj(gv), __ldg(dY + (long)c * rows + r));
             }
         }
     }
     __syncthreads();
 #pragma unroll
-    for (int y = 0; y < FA_T / 16; y++) {
-        const long r = r0 + warp + 16 * y;
+    for (int y = 0; y < 4; y++) {
+        const long r = r0 + warp + FA_T / 4 * y;
         if (r >= rows) continue;
 #pragma unroll
-        for (int h = 0; h < 2; h++) {
+        for (int h = 0; h < FA_T / 32; h++) {
             const int c = c0 + 32 * h + lane;
-            if (c < nch) dF[r * nch + c] = t[32 * h + lane][warp + 16 * y];
+            if (c < nch) dF[r * nch + c] = t[32 * h + lane][warp + FA_T / 4 * y];
         }
     }
 }
 
-// dY[c][s][r] = scale * sum_q (G_rq + conj(G_qr)) Y[c][s][q].  A block takes 64
-// elements r of one channel and XA_TILES tiles of 64 spectra; a thread holds 8
-// spectra x 4 elements, summed over q in increasing order with the multiply-adds
-// of a complex product in turn, two lanes of an f32x2 fma each.  Chunks of 64 q
-// of H = G + G^H and of Y go through shared memory (H stays there over the
-// block's spectra when one chunk holds all of it).  Bound by the FP32 pipe: per
-// pair of q a warp issues 128 packed fmas against 16 shared-memory wavefronts (one
-// output per thread and 16 x 16 tiles: two 8-byte loads per four fmas).
+// dY[c][s][r] = scale * sum_q (G_rq + conj(G_qr)) Y[c][s][q].  A block takes R
+// elements r of one channel and `tiles` tiles of S spectra; a thread holds SP spectra x
+// 4 elements, summed over q in increasing order with the multiply-adds of a complex
+// product in turn, two lanes of an f32x2 fma each.  Chunks of R elements q of
+// H = G + G^H and of Y go through shared memory (H stays there over the block's
+// spectra when one chunk holds all of it).  With 8 spectra a thread it is bound by the
+// FP32 pipe: per pair of q a warp issues 128 packed fmas against 16 shared-memory
+// wavefronts (one output per thread and 16 x 16 tiles: two 8-byte loads per four fmas).
 // NE=64, Nch=512, Nsp=2048: 0.95 ms (36 TFLOP/s, 47 % of the FP32 rate), 2.44 before.
-constexpr int XA_T = 64, XA_TILES = 4, XA_THREADS = 128;
-constexpr int XA_YS = XA_T + 2;  // float2 per staged row of Y (16-byte rows, skewed banks)
-constexpr size_t XA_SMEM = sizeof(float2) * ((size_t)XA_T * XA_T + (size_t)XA_T * XA_YS);
+constexpr int XA_THREADS = 128;
+template <int R, int SP>
+struct XaCfg {
+    static constexpr int TX = R / 4, TY = XA_THREADS / TX;  // threads over elements, spectra
+    static constexpr int S = SP * TY;
+    static constexpr int YS = R + 2;  // float2 per staged row of Y (16-byte rows, skewed banks)
+    static constexpr size_t SMEM = sizeof(float2) * ((size_t)R * R + (size_t)S * YS);
+};
 
+template <int R, int SP>
 __global__ void __launch_bounds__(XA_THREADS, 4)
-    xengine_adjoint_kernel(int ne, int nsp, const float2 *__restrict__ G,
+    xengine_adjoint_kernel(int ne, int nsp, int tiles, const float2 *__restrict__ G,
                            const float2 *__restrict__ Y, float2 *__restrict__ dY, float scale)
 {
+    using C = XaCfg<R, SP>;
     extern __shared__ float4 xa_smem[];
     float2 *sh = reinterpret_cast<float2 *>(xa_smem);  // [q][r]
-    float2 *sy = sh + XA_T * XA_T;                     // [s][q], XA_YS per row
-    const int c = blockIdx.z, r0 = blockIdx.x * XA_T, tid = threadIdx.x;
+    float2 *sy = sh + R * R;                           // [s][q], YS per row
+    const int c = blockIdx.z, r0 = blockIdx.x * R, tid = threadIdx.x;
     const float2 *Gc = G + (long)c * ne * ne;
     const float2 *Yc = Y + (long)c * nsp * ne;
     float2 *dYc = dY + (long)c * nsp * ne;
-    const int tr = tid & 15, ts = tid >> 4;  // elements 2 tr + {0, 1, 32, 33}, spectra 8 ts + i
-    const int nchunk = (ne + XA_T - 1) / XA_T;
+    // elements 2 tr + {0, 1, R/2, R/2 + 1}, spectra ts + TY i
+    const int tr = tid % C::TX, ts = tid / C::TX;
+    const int nchunk = (ne + R - 1) / R;
     // H[q0 + q][r0 + r] = G_rq + conj(G_qr), zero past NE
     auto load_h = [&](int q0) {
-        for (int i = tid; i < XA_T * XA_T; i += XA_THREADS) {
-            const int q = i >> 6, r = i & 63;
+        for (int i = tid; i < R * R; i += XA_THREADS) {
+            const int q = i / R, r = i % R;
             float2 h = make_float2(0.f, 0.f);
             if (r0 + r < ne && q0 + q < ne) h = __ldg(Gc + (long)(q0 + q) * ne + r0 + r);  // G_rq
             sh[i] = h;
         }
         __syncthreads();
-        for (int i = tid; i < XA_T * XA_T; i += XA_THREADS) {
-            const int r = i >> 6, q = i & 63;
+        for (int i = tid; i < R * R; i += XA_THREADS) {
+            const int r = i / R, q = i % R;
             if (r0 + r < ne && q0 + q < ne) {
                 const float2 b = __ldg(Gc + (long)(r0 + r) * ne + q0 + q);  // G_qr
-                float2 &h = sh[q * XA_T + r];
+                float2 &h = sh[q * R + r];
                 h = make_float2(h.x + b.x, h.y - b.y);
             }
         }
     };
     auto load_y = [&](int s0, int q0) {
 #pragma unroll 8
-        for (int i = tid; i < XA_T * XA_T; i += XA_THREADS) {
-            const int s = i >> 6, q = i & 63;
-            sy[s * XA_YS + q] = s0 + s < nsp && q0 + q < ne ? __ldg(Yc + (long)(s0 + s) * ne + q0 + q)
-                                                            : make_float2(0.f, 0.f);
+        for (int i = tid; i < C::S * R; i += XA_THREADS) {
+            const int s = i / R, q = i % R;
+            sy[s * C::YS + q] = s0 + s < nsp && q0 + q < ne
+                                    ? __ldg(Yc + (long)(s0 + s) * ne + q0 + q)
+                                    : make_float2(0.f, 0.f);
         }
     };
     if (nchunk == 1) load_h(0);
-    for (int t = 0; t < XA_TILES; t++) {
-        const int s0 = (blockIdx.y * XA_TILES + t) * XA_T;
+    for (int t = 0; t < tiles; t++) {
+        const int s0 = (blockIdx.y * tiles + t) * C::S;
         if (s0 >= nsp) break;
-        float2 acc[8][4];
+        float2 acc[SP][4];
 #pragma unroll
-        for (int i = 0; i < 8; i++)
+        for (int i = 0; i < SP; i++)
 #pragma unroll
             for (int j = 0; j < 4; j++) acc[i][j] = make_float2(0.f, 0.f);
         for (int k = 0; k < nchunk; k++) {
             __syncthreads();  // the staged chunks have been read
-            if (nchunk > 1) load_h(k * XA_T);
-            load_y(s0, k * XA_T);
+            if (nchunk > 1) load_h(k * R);
+            load_y(s0, k * R);
             __syncthreads();
-            const int nq = min(XA_T, (ne - k * XA_T + 1) & ~1);
+            const int nq = min(R, (ne - k * R + 1) & ~1);
 #pragma unroll 2
             for (int q = 0; q < nq; q += 2) {
                 float4 h[2][2];
@@ -284,10 +293,10 @@ __global__ void __launch_bounds__(XA_THREADS, 4)
                 for (int u = 0; u < 2; u++)
 #pragma unroll
                     for (int v = 0; v < 2; v++)
-                        h[u][v] = *reinterpret_cast<const float4 *>(sh + (q + u) * XA_T + 32 * v + 2 * tr);
+                        h[u][v] = *reinterpret_cast<const float4 *>(sh + (q + u) * R + R / 2 * v + 2 * tr);
 #pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    const float4 y4 = *reinterpret_cast<const float4 *>(sy + (8 * ts + i) * XA_YS + q);
+                for (int i = 0; i < SP; i++) {
+                    const float4 y4 = *reinterpret_cast<const float4 *>(sy + (ts + C::TY * i) * C::YS + q);
 #pragma unroll
                     for (int u = 0; u < 2; u++) {
                         const float2 y = u ? make_float2(y4.z, y4.w) : make_float2(y4.x, y4.y);
@@ -305,17 +314,52 @@ __global__ void __launch_bounds__(XA_THREADS, 4)
             }
         }
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const int s = s0 + 8 * ts + i;
+        for (int i = 0; i < SP; i++) {
+            const int s = s0 + ts + C::TY * i;
             if (s >= nsp) continue;
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                const int r = r0 + 32 * (j >> 1) + 2 * tr + (j & 1);
+                const int r = r0 + R / 2 * (j >> 1) + 2 * tr + (j & 1);
                 if (r < ne)
                     dYc[(long)s * ne + r] = make_float2(acc[i][j].x * scale, acc[i][j].y * scale);
             }
         }
     }
+}
+
+template <int R, int SP>
+static mdt_status xengine_adjoint_launch(int ne, int nch, int nsp, const float2 *G, const float2 *Y,
+                                         float2 *dY, float scale, cudaStream_t stream)
+{
+    using C = XaCfg<R, SP>;
+    // up to four tiles to a block (they share its H) while that leaves four blocks an SM
+    const long gx = cdiv(ne, R), all = cdiv(nsp, C::S);
+    const int tiles = (int)std::max<long>(1, std::min<long>(4, gx * all * nch / (4L * sm_count())));
+    cudaError_t e = cudaFuncSetAttribute(xengine_adjoint_kernel<R, SP>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
+    if (e != cudaSuccess) return cuda_status(e, "xengine_adjoint_f32 smem attribute");
+    const dim3 grid((unsigned)gx, (unsigned)cdiv(all, tiles), (unsigned)nch);
+    xengine_adjoint_kernel<R, SP><<<grid, XA_THREADS, C::SMEM, stream>>>(ne, nsp, tiles, G, Y, dY,
+                                                                         scale);
+    return launch_status("xengine_adjoint_kernel");
+}
+
+// The tile by the elements and spectra that it would leave empty.  Up to 16 elements
+// 16 x 64 spectra (NE=12, Nch=512, Nsp=1000: 40 us; 32 x 128 68, 64 x 64 143).  Up to 32
+// spectra 32 x 32 (NE=64, Nsp=30: 31 us; 32 x 128 69, 64 x 64 50), and up to 64 for up to
+// 32 elements.  Otherwise 32 x 128 (NE=28, Nsp=1000: 129 us, 64 x 64 249; NE=96 1175
+// and 1715, NE=192 4437 and 5078), but for 33 to 64 elements, whose H one 64 x 64 tile
+// keeps (NE=64, Nsp=1000: 502 us, 32 x 128 541), and for too few spectra (NE=128,
+// Nsp=60: 168 and 262).
+static mdt_status xengine_adjoint(int ne, int nch, int nsp, const float2 *G, const float2 *Y,
+                                  float2 *dY, float scale, cudaStream_t stream)
+{
+    if (ne <= 16) return xengine_adjoint_launch<16, 2>(ne, nch, nsp, G, Y, dY, scale, stream);
+    if (nsp <= (ne <= 32 ? 64 : 32))
+        return xengine_adjoint_launch<32, 2>(ne, nch, nsp, G, Y, dY, scale, stream);
+    if (ne > 32 && (ne <= 64 || nsp <= 64))
+        return xengine_adjoint_launch<64, 8>(ne, nch, nsp, G, Y, dY, scale, stream);
+    return xengine_adjoint_launch<32, 8>(ne, nch, nsp, G, Y, dY, scale, stream);
 }
 
 // Partial tap gradients: split p of the (spectrum, element) rows.
@@ -472,14 +516,8 @@ MDT_API mdt_status mdt_xengine_adjoint_f32(int ne, int nch, int nsp, const void 
     if (!G || !Y || !dY || ne < 1 || nch < 1 || nsp < 1 || nch > 65535)
         return mdt::invalid("xengine_adjoint_f32: bad arguments");
     if (mdt::cdiv(nsp, 16) > 65535) return mdt::invalid("xengine_adjoint_f32: Nsp too large");
-    dim3 grid((unsigned)mdt::cdiv(ne, mdt::XA_T), (unsigned)mdt::cdiv(nsp, mdt::XA_T * mdt::XA_TILES),
-              (unsigned)nch);
-    cudaError_t e = cudaFuncSetAttribute(mdt::xengine_adjoint_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mdt::XA_SMEM);
-    if (e != cudaSuccess) return mdt::cuda_status(e, "xengine_adjoint_f32 smem attribute");
-    mdt::xengine_adjoint_kernel<<<grid, mdt::XA_THREADS, mdt::XA_SMEM, stream>>>(
-        ne, nsp, (const float2 *)G, (const float2 *)Y, (float2 *)dY, scale);
-    return mdt::launch_status("xengine_adjoint_kernel");
+    return mdt::xengine_adjoint(ne, nch, nsp, (const float2 *)G, (const float2 *)Y, (float2 *)dY,
+                                scale, stream);
 }
 
 MDT_API mdt_status mdt_apply_gains(int ne, int nch, int nsp, const void *X, const void *gains,
@@ -526,9 +564,16 @@ MDT_API mdt_status mdt_gain_adjoint(int ne, int nch, int nsp, const void *dY, co
     }
     if (dF) {
         const long rows = (long)nsp * ne;
-        dim3 grid((unsigned)mdt::cdiv(rows, mdt::FA_T), (unsigned)mdt::cdiv(nch, mdt::FA_T));
-        mdt::fout_adjoint_kernel<<<grid, dim3(32, 16), 0, stream>>>(
-            ne, nch, rows, (const float2 *)dY, (const float2 *)gains, (float2 *)dF);
+        // tiles of 32 where those of 64 would leave SMs without a pair of blocks
+        auto launch = [&](auto kern, int t) {
+            const dim3 grid((unsigned)mdt::cdiv(rows, t), (unsigned)mdt::cdiv(nch, t));
+            kern<<<grid, dim3(32, t / 4), 0, stream>>>(ne, nch, rows, (const float2 *)dY,
+                                                       (const float2 *)gains, (float2 *)dF);
+        };
+        if (mdt::cdiv(rows, 64) * mdt::cdiv(nch, 64) < 2L * mdt::sm_count())
+            launch(mdt::fout_adjoint_kernel<32>, 32);
+        else
+            launch(mdt::fout_adjoint_kernel<64>, 64);
         return mdt::launch_status("fout_adjoint_kernel");
     }
     return MDT_SUCCESS;

@@ -1,0 +1,43 @@
+"""Adjoint kernels at the edges of their tiles: X-engine adjoint tiles of 16, 32 and 64
+elements with few and many spectra, the reorder's adjoint in tiles of 32 and 64 (an
+exact transpose without gains)."""
+import numpy as np
+import pytest
+import torch
+
+from adjref import crandn
+
+pytestmark = pytest.mark.gpu
+
+
+def dev(a):
+    return torch.from_numpy(np.ascontiguousarray(a)).cuda()
+
+
+def rel(a, b):
+    return float(np.linalg.norm((a - b).ravel()) / np.linalg.norm(b.ravel()))
+
+
+@pytest.mark.parametrize("ne", [1, 15, 16, 17, 32, 33, 64, 65, 96, 129])
+@pytest.mark.parametrize("nch,nsp", [(3, 1), (2, 32), (2, 33), (3, 64), (2, 65), (1, 300), (700, 35)])
+def test_xengine_adjoint_tiles(mdt, cuda, ne, nch, nsp):
+    if nch * ne * nsp > 2e6:
+        ne = 31  # many channels: several spectrum tiles to a block
+    rng = np.random.default_rng(ne * 1009 + nsp)
+    G = crandn(rng, nch, ne, ne).astype(np.complex64)
+    Y = crandn(rng, nch, nsp, ne).astype(np.complex64)
+    dY = torch.full((nch, nsp, ne), float("nan"), dtype=torch.complex64, device="cuda")
+    mdt.xengine_adjoint_f32(ne, nch, nsp, dev(G), dev(Y), dY, 0.5)
+    Gm = np.transpose(G.astype(np.complex128), (0, 2, 1))
+    H = Gm + np.conj(np.transpose(Gm, (0, 2, 1)))
+    want = 0.5 * np.matmul(Y.astype(np.complex128), np.transpose(H, (0, 2, 1)))
+    # an FP32 chain of 2 NE fmas: 2^-24 of a random walk's length, and H's rounding
+    assert rel(dY.cpu().numpy(), want) < 2.0 ** -24 * (2 + 2 * np.sqrt(2 * ne))
+
+
+@pytest.mark.parametrize("ne,nch,nsp", [(3, 40, 7), (5, 64, 33), (33, 300, 100), (64, 512, 65)])
+def test_reorder_adjoint_tiles(mdt, cuda, ne, nch, nsp):
+    dY = dev(crandn(np.random.default_rng(nch), nch, nsp, ne).astype(np.complex64))
+    dF = torch.full((nsp, ne, nch), float("nan"), dtype=torch.complex64, device="cuda")
+    mdt.gain_adjoint(ne, nch, nsp, dY, gains=None, dF=dF)
+    assert torch.equal(torch.view_as_real(dF), torch.view_as_real(dY.permute(1, 2, 0)))
