@@ -12,6 +12,7 @@
 //   mdt_fft_c2c direction +1) and
 //   grad(W)[i][k] = sum_{s,e} Re(grad(P)[s][e][k] * conj(in[s+i][e][k])).
 #include <algorithm>
+#include <type_traits>
 
 #include "mdt_common.cuh"
 
@@ -387,15 +388,15 @@ __global__ void pfb_tap_grad_partial_kernel(int nch, int ntaps, int ne, int nsp,
 }
 
 // NT = 4 or 8 taps at once: part[p][i][k] as above.  A thread owns VEC
-// channels and walks runs of TG_RUN spectra of one element, so that every
+// channels and walks runs of `len` spectra of one element, so that every
 // gradient value and (but for the NT-1 spectra of a run's lead-in) every
 // sample is read once; the samples of the NT taps rotate through registers.
 // The runs are dealt to the TG_PH warps of a block and to the splits in turn;
 // each thread's sums are compensated FP32, combined in double in a fixed
 // order.  Bound by the FP32 pipe (10 operations a product; 145 us at NE=64,
 // Nch=512, 4 taps, Nsp=2048) and by latency: 265 us there, 3328 us with sums
-// in double.
-constexpr int TG_PH = 16, TG_RUN = 32;
+// in double.  With 8 taps 455 us (522 with a test on each spectrum of a run).
+constexpr int TG_PH = 16, TG_RUN = 32;  // warps, longest run
 
 template <int VEC>
 __device__ __forceinline__ void load_iq(const char2 *p, float (&re)[VEC], float (&im)[VEC])
@@ -414,25 +415,26 @@ __device__ __forceinline__ void load_iq(const char2 *p, float (&re)[VEC], float 
 }
 
 template <int NT, int VEC, class Sum>
-__device__ __forceinline__ bool tap_sums(int nch, int ne, int nsp, int k, long first, long stride,
+__device__ __forceinline__ bool tap_sums(int nch, int ne, int nsp, int len, int k, long first, long stride,
                                          const float2 *__restrict__ gP,
                                          const char2 *__restrict__ iq, double (&out)[NT][VEC])
 {
     Sum acc[NT][VEC];
-    const long nruns = (long)ne * ((nsp + TG_RUN - 1) / TG_RUN);
+    const long nruns = (long)ne * ((nsp + len - 1) / len);
     const long spec = (long)ne * nch;
     for (long t = first; t < nruns; t += stride) {
         const int run = (int)(t / ne), e = (int)(t - (long)run * ne);
-        const int s0 = run * TG_RUN, s1 = min(nsp, s0 + TG_RUN);
+        const int s0 = run * len, s1 = min(nsp, s0 + len);
         const float2 *g = gP + (long)s0 * spec + (long)e * nch + k;
         const char2 *x = iq + (long)s0 * spec + (long)e * nch + k;
         float xr[NT][VEC], xi[NT][VEC];  // spectrum s in slot (s - s0) % NT
 #pragma unroll
         for (int i = 0; i < NT - 1; i++) load_iq<VEC>(x + i * spec, xr[i], xi[i]);
-        for (int s = s0; s < s1; s += NT) {
+        // NT spectra from s on; without a test on each, their loads are all issued ahead
+        auto group = [&](int s, auto full) {
 #pragma unroll
             for (int u = 0; u < NT; u++) {
-                if (s + u < s1) {
+                if (decltype(full)::value || s + u < s1) {
                     float2 gv[VEC];
                     load_c64<VEC>(g + (long)(s + u - s0) * spec, gv);
                     load_iq<VEC>(x + (long)(s + u - s0 + NT - 1) * spec, xr[(u + NT - 1) % NT],
@@ -446,7 +448,10 @@ __device__ __forceinline__ bool tap_sums(int nch, int ne, int nsp, int k, long f
                         }
                 }
             }
-        }
+        };
+        int s = s0;
+        for (; s + NT <= s1; s += NT) group(s, std::true_type());
+        if (s < s1) group(s, std::false_type());
     }
     bool ok = true;
 #pragma unroll
@@ -460,17 +465,17 @@ __device__ __forceinline__ bool tap_sums(int nch, int ne, int nsp, int k, long f
 }
 
 template <int NT, int VEC>
-__global__ void __launch_bounds__(32 * TG_PH)
-    pfb_tap_grad_all_kernel(int nch, int ne, int nsp, int nsplit, const float2 *__restrict__ gP,
-                            const char2 *__restrict__ iq, double *__restrict__ part)
+__global__ void __launch_bounds__(32 * TG_PH, NT * VEC <= 8 ? 2 : 1)
+    pfb_tap_grad_all_kernel(int nch, int ne, int nsp, int len, int nsplit,
+                            const float2 *__restrict__ gP, const char2 *__restrict__ iq, double *__restrict__ part)
 {
     __shared__ double red[TG_PH][32 * VEC];
     const int k = (blockIdx.x * 32 + threadIdx.x) * VEC;
     const int ph = threadIdx.y, p = blockIdx.y;
     const long first = (long)p * TG_PH + ph, stride = (long)nsplit * TG_PH;
     double sum[NT][VEC] = {};
-    if (k < nch && !tap_sums<NT, VEC, Sum2>(nch, ne, nsp, k, first, stride, gP, iq, sum))
-        tap_sums<NT, VEC, SumD>(nch, ne, nsp, k, first, stride, gP, iq, sum);
+    if (k < nch && !tap_sums<NT, VEC, Sum2>(nch, ne, nsp, len, k, first, stride, gP, iq, sum))
+        tap_sums<NT, VEC, SumD>(nch, ne, nsp, len, k, first, stride, gP, iq, sum);
     const int tid = ph * 32 + threadIdx.x;
 #pragma unroll
     for (int i = 0; i < NT; i++) {
@@ -595,16 +600,20 @@ MDT_API mdt_status mdt_pfb_tap_grad(int ne, int nch, int ntaps, int nsp, const v
         // two channels per thread (16-byte gradients, 4-byte samples) where Nch is
         // even and the buffers are aligned for it
         const bool v2 = nch % 2 == 0 && ((uintptr_t)gradP & 15) == 0 && ((uintptr_t)iq & 3) == 0;
-        const long runs = (long)ne * mdt::cdiv(nsp, mdt::TG_RUN);
         // two blocks of 16 warps fit an SM: as many splits as fill the GPU once
         // (64 splits, 1.7 waves at Nch 512: 296 us against 265)
         const long once = 2L * mdt::sm_count() / mdt::cdiv(nch, 32 * (v2 ? 2 : 1));
+        // shorter runs where those of 32 spectra are too few for the warps of a wave
+        // (NE=28, Nch=512, Nsp=30: 14 us, with runs of 32 25 us)
+        int len = mdt::TG_RUN;
+        while (len > 8 && ne * mdt::cdiv(nsp, len) < once * mdt::TG_PH) len /= 2;
+        const long runs = ne * mdt::cdiv(nsp, len);
         nsplit = (int)std::max<long>(1, std::min<long>(std::min<long>(nsplit, once),
                                                        mdt::cdiv(runs, mdt::TG_PH)));
         auto launch = [&](auto kern, int vec) {
             const dim3 grid((unsigned)mdt::cdiv(nch, 32 * vec), (unsigned)nsplit);
             kern<<<grid, dim3(32, mdt::TG_PH), 0, stream>>>(
-                nch, ne, nsp, nsplit, (const float2 *)gradP, (const char2 *)iq, (double *)workspace);
+                nch, ne, nsp, len, nsplit, (const float2 *)gradP, (const char2 *)iq, (double *)workspace);
         };
         if (ntaps == 4) {
             if (v2) launch(mdt::pfb_tap_grad_all_kernel<4, 2>, 2);

@@ -1,6 +1,6 @@
 """Adjoint kernels at the edges of their tiles: X-engine adjoint tiles of 16, 32 and 64
 elements with few and many spectra, the reorder's adjoint in tiles of 32 and 64 (an
-exact transpose without gains)."""
+exact transpose without gains), tap gradients over short and long runs."""
 import numpy as np
 import pytest
 import torch
@@ -41,3 +41,24 @@ def test_reorder_adjoint_tiles(mdt, cuda, ne, nch, nsp):
     dF = torch.full((nsp, ne, nch), float("nan"), dtype=torch.complex64, device="cuda")
     mdt.gain_adjoint(ne, nch, nsp, dY, gains=None, dF=dF)
     assert torch.equal(torch.view_as_real(dF), torch.view_as_real(dY.permute(1, 2, 0)))
+
+
+@pytest.mark.parametrize("ntaps", [4, 8])
+@pytest.mark.parametrize("ne,nch,nsp", [(1, 32, 2), (3, 256, 16), (3, 255, 33), (20, 512, 70),
+                                        (64, 128, 129)])
+def test_tap_grad_runs(mdt, cuda, ntaps, ne, nch, nsp):
+    rng = np.random.default_rng(nsp + ntaps)
+    gP = crandn(rng, nsp, ne, nch).astype(np.complex64)
+    iq = rng.integers(-128, 128, (nsp + ntaps - 1, ne, nch, 2)).astype(np.int8)
+    gW = torch.full((ntaps, nch), float("nan"), dtype=torch.float32, device="cuda")
+    ws = torch.empty(ntaps * nch * 64, dtype=torch.float64, device="cuda")
+    mdt.pfb_tap_grad(ne, nch, ntaps, nsp, dev(gP), dev(iq), gW, ws)
+    x = iq[..., 0] + 1j * iq[..., 1].astype(np.float64)
+    want = np.stack([np.einsum("sek,sek->k", gP.astype(np.complex128), np.conj(x[i:i + nsp])).real
+                     for i in range(ntaps)])
+    # sums in twice the working precision, rounded once to FP32 (cancelling sums: of
+    # the products' own size)
+    size = np.stack([np.einsum("sek,sek->k", np.abs(gP), np.abs(x[i:i + nsp]))
+                     for i in range(ntaps)])
+    got = gW.cpu().numpy()
+    assert np.all(np.abs(got - want) <= 2.0 ** -24 * np.abs(want) + 2.0 ** -40 * size)
