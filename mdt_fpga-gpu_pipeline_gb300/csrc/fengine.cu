@@ -25,12 +25,12 @@
 
 namespace mdt {
 
-// Rows (elements) per block of the FP32 F-engine.
-// Small blocks let several blocks share an SM, so one block's sample loads
-// overlap another's FFT passes and barriers.
-#ifndef MDT_FENG_ROWS
-#define MDT_FENG_ROWS 8
-#endif
+// (Spectrum, element) rows per block of the FP32 F-engine, of whatever spectrum, so
+// that only the last block has rows to spare.  Small blocks let several blocks share
+// an SM, so one block's sample loads overlap another's FFT passes and barriers.
+// Blocks of 8 rows; where those would leave SMs without a pair of blocks, of 4 rows with
+// N/8 threads (up to 256) each, which wait for one chain of tap loads, not two (48
+// rows of Nch 256, 8 taps: 4.1 us against 5.8; 320 rows of Nch 2048 9.6 and 15.2).
 // Threads per SM the register budget is sized for (64K registers / this).
 #ifndef MDT_FENG_SM_THREADS
 #define MDT_FENG_SM_THREADS 1024
@@ -44,14 +44,15 @@ namespace mdt {
 // taps, FP32: 101 us, with N/16 109; of Nch 128 172 and 182).
 constexpr int feng_tpr(int n) { return n < 256 ? n / 8 : n / 16; }
 
-template <int N>
+template <int N, int R>
 struct FengCfg {
-    static constexpr int TPR = feng_tpr(N);
+    static constexpr int TPR = R == 8 ? feng_tpr(N) : N / 8 < 256 ? N / 8 : N / 16 > 256 ? N / 16 : 256;
     static constexpr int RMAX = (1024 / TPR) < 1 ? 1 : 1024 / TPR;
-    static constexpr int ROWS = MDT_FENG_ROWS < RMAX ? MDT_FENG_ROWS : RMAX;
+    static constexpr int ROWS = R < RMAX ? R : RMAX;
     static constexpr int THREADS = ROWS * TPR;
     // resident blocks per SM requested from the register allocator
-    static constexpr int MINB = (MDT_FENG_SM_THREADS / THREADS) < 1 ? 1 : (MDT_FENG_SM_THREADS / THREADS);
+    static constexpr int MINB =
+        MDT_FENG_SM_THREADS / THREADS < 1 ? 1 : MDT_FENG_SM_THREADS / THREADS;
     static constexpr int RSTRIDE = fft::Shape<N>::PADN + 4;  // float2 per row (bank skew)
     static constexpr size_t SMEM = sizeof(float2) * (size_t)RSTRIDE * ROWS;
 };
@@ -60,7 +61,7 @@ struct FengArgs {
     const char2 *hist;  // first nhist spectra (may be null when nhist == 0)
     const char2 *iq;    // remaining spectra
     int nhist;
-    int ne, ntaps, nsp, ngroups;
+    int ne, ntaps, nsp;
     const float *win;
     const float2 *tw;
     float2 *X;
@@ -70,28 +71,26 @@ struct FengArgs {
 // order, padded): each work item is 8 consecutive channels of one row, read
 // as one 16-byte int8 I/Q vector and two float4 window vectors per tap;
 // accumulation is fmaf from zero in increasing tap order.  Row r of the block
-// is (spectrum s0, element e0 + r), or with SPECTRA_ROWS (spectrum s0 + r,
-// element e0); rows past NE or Nsp are zero.
-template <int N, int ROWS, int THREADS, bool SPECTRA_ROWS = false>
-__device__ __forceinline__ void pfb_rows_to_smem(const FengArgs &a, int s0, int e0, float2 *smem,
+// is row row0 + r*step of the Nsp*NE (spectrum, element) rows; rows past the
+// last are zero.
+template <int N, int ROWS, int THREADS>
+__device__ __forceinline__ void pfb_rows_to_smem(const FengArgs &a, long row0, int step, float2 *smem,
                                                  int rstride)
 {
     constexpr int ITEMS = ROWS * (N / 8);
-    const long rowlen = (long)a.ne * N;
+    const long rows = (long)a.nsp * a.ne, hrows = (long)a.nhist * a.ne;
     for (int it = threadIdx.x; it < ITEMS; it += THREADS) {
         const int r = it / (N / 8);
         const int c0 = (it - r * (N / 8)) * 8;
-        const int e = SPECTRA_ROWS ? e0 : e0 + r;
-        const int s = SPECTRA_ROWS ? s0 + r : s0;
+        const long row = row0 + (long)r * step;
         float re[8], im[8];
 #pragma unroll
         for (int k = 0; k < 8; k++) re[k] = im[k] = 0.0f;
-        if (e < a.ne && s < a.nsp) {
+        if (row < rows) {
             for (int i = 0; i < a.ntaps; i++) {
-                const int sp = s + i;
-                const char2 *src = (sp < a.nhist) ? a.hist + (long)sp * rowlen
-                                                  : a.iq + (long)(sp - a.nhist) * rowlen;
-                const int4 raw = __ldg(reinterpret_cast<const int4 *>(src + (long)e * N + c0));
+                const long in = row + (long)i * a.ne;
+                const char2 *src = in < hrows ? a.hist + in * N : a.iq + (in - hrows) * N;
+                const int4 raw = __ldg(reinterpret_cast<const int4 *>(src + c0));
                 const float4 w0 = __ldg(reinterpret_cast<const float4 *>(a.win + (long)i * N + c0));
                 const float4 w1 =
                     __ldg(reinterpret_cast<const float4 *>(a.win + (long)i * N + c0 + 4));
@@ -115,31 +114,29 @@ __device__ __forceinline__ void pfb_rows_to_smem(const FengArgs &a, int s0, int 
     }
 }
 
-template <int N>
-__global__ void __launch_bounds__(FengCfg<N>::THREADS, FengCfg<N>::MINB) fengine_f32_kernel(FengArgs a)
+template <int N, int R>
+__global__ void __launch_bounds__(FengCfg<N, R>::THREADS, FengCfg<N, R>::MINB)
+    fengine_f32_kernel(FengArgs a)
 {
-    using C = FengCfg<N>;
+    using C = FengCfg<N, R>;
     extern __shared__ float2 fsm[];
-    const long blk = blockIdx.x;
-    const int s = (int)(blk / a.ngroups);
-    const int e0 = (int)(blk - (long)s * a.ngroups) * C::ROWS;
+    const long row0 = (long)blockIdx.x * C::ROWS, rows = (long)a.nsp * a.ne;
     const int lrow = threadIdx.x / C::TPR;
     const int t = threadIdx.x - lrow * C::TPR;
 
-    pfb_rows_to_smem<N, C::ROWS, C::THREADS>(a, s, e0, fsm, C::RSTRIDE);
+    pfb_rows_to_smem<N, C::ROWS, C::THREADS>(a, row0, 1, fsm, C::RSTRIDE);
     __syncthreads();
     auto none_load = [](int) { return make_float2(0.f, 0.f); };
     auto none_store = [](int, float2) {};
     fft::transform_row<N, C::TPR, false, false>(fsm + (size_t)lrow * C::RSTRIDE, t, a.tw,
                                                 none_load, none_store);
 
-    // corner turn: ROWS contiguous elements per channel
-    const int nrow = min(C::ROWS, a.ne - e0);
-    float2 *dst = a.X + (long)s * a.ne + e0;
-    const long cstride = (long)a.nsp * a.ne;
+    // corner turn: ROWS contiguous (spectrum, element) rows per channel
+    const int nrow = (int)min((long)C::ROWS, rows - row0);
+    float2 *dst = a.X + row0;
     for (int k = threadIdx.x; k < N * C::ROWS; k += C::THREADS) {
         const int c = k / C::ROWS, r = k - c * C::ROWS;
-        if (r < nrow) dst[(long)c * cstride + r] = fsm[(size_t)r * C::RSTRIDE + fft::pad(c)];
+        if (r < nrow) dst[(long)c * rows + r] = fsm[(size_t)r * C::RSTRIDE + fft::pad(c)];
     }
 }
 
@@ -402,7 +399,7 @@ __device__ __forceinline__ void fengine_block8(const FengArgs &a, const Block8 &
                                               fill_tw);
     } else {
         fill_tw();
-        pfb_rows_to_smem<N, SB8, C::THREADS, true>(a, b.s0, b.e, fsm, C::RSTRIDE);
+        pfb_rows_to_smem<N, SB8, C::THREADS>(a, (long)b.s0 * a.ne + b.e, a.ne, fsm, C::RSTRIDE);
     }
     __syncthreads();
     const int lrow = threadIdx.x / C::TPR;
@@ -654,7 +651,6 @@ __global__ void __launch_bounds__(FengBCfg<N>::THREADS, FengBCfg<N>::MINB)
         a.ne = jb.ne;
         a.ntaps = NT;
         a.nsp = jb.nsp;
-        a.ngroups = 0;
         a.win = jb.win;
         a.tw = tw;
         a.X = nullptr;
@@ -802,7 +798,6 @@ static FengArgs make_args(int ne, int ntaps, int nsp, const int8_t *hist, int nh
     a.nsp = nsp;
     a.win = win;
     a.X = nullptr;
-    a.ngroups = 0;
     a.tw = nullptr;
     return a;
 }
@@ -911,24 +906,30 @@ mdt_status fengine_c64b_given_twiddles(int ne, int nch, int ntaps, int nsp, cons
 }
 
 // ------------------------------------------------------------------------
-template <int N>
-static mdt_status launch_feng(FengArgs a, cudaStream_t stream)
+template <int N, int R>
+static mdt_status launch_feng_rows(FengArgs a, cudaStream_t stream)
 {
-    using C = FengCfg<N>;
+    using C = FengCfg<N, R>;
     mdt_status st;
     a.tw = fft_twiddles(N, &st);
     if (!a.tw) return st;
     if (C::SMEM > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(fengine_f32_kernel<N>,
+        cudaError_t e = cudaFuncSetAttribute(fengine_f32_kernel<N, R>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)C::SMEM);
         if (e != cudaSuccess) return cuda_status(e, "fengine smem attribute");
     }
-    a.ngroups = (int)cdiv(a.ne, C::ROWS);
-    long blocks = (long)a.nsp * a.ngroups;
+    const long blocks = cdiv((long)a.nsp * a.ne, C::ROWS);
     if (blocks > 0x7fffffffL) return invalid("fengine: grid too large");
-    fengine_f32_kernel<N><<<(unsigned)blocks, C::THREADS, C::SMEM, stream>>>(a);
+    fengine_f32_kernel<N, R><<<(unsigned)blocks, C::THREADS, C::SMEM, stream>>>(a);
     return launch_status("fengine_f32_kernel");
+}
+
+template <int N>
+static mdt_status launch_feng(const FengArgs &a, cudaStream_t stream)
+{
+    return cdiv((long)a.nsp * a.ne, 8) < 2L * sm_count() ? launch_feng_rows<N, 4>(a, stream)
+                                                         : launch_feng_rows<N, 8>(a, stream);
 }
 
 mdt_status fengine_f32(int ne, int nch, int ntaps, int nsp, const int8_t *hist, int nhist,
