@@ -406,8 +406,10 @@ __device__ __forceinline__ void fengine_block8(const FengArgs &a, const Block8 &
     const int t = threadIdx.x - lrow * C::TPR;
     auto none_load = [](int) { return make_float2(0.f, 0.f); };
     auto none_store = [](int, float2) {};
-    fft::transform_row_tws<N, C::TPR, false, false>(fsm + (size_t)lrow * C::RSTRIDE, t, tws,
-                                                    none_load, none_store);
+    constexpr bool kRowSync = NT > 0 && N >= 64;
+    fft::transform_row_tws<N, C::TPR, false, false, kRowSync>(fsm + (size_t)lrow * C::RSTRIDE, t, tws,
+                                                              none_load, none_store);
+    if (kRowSync) __syncthreads();
 }
 
 // FP32 output in the 8-spectrum blocked layout of the plan's FP32 path (XB,
@@ -471,8 +473,9 @@ __device__ __forceinline__ void fengine_units(int u, int step, int nunits, const
             unit(un, a, b);
             stage_rows_async<N, NT, C::THREADS>(a, b.s0, b.e, stage);
         }
-        fft::transform_row_tws<N, C::TPR, false, false>(fsm + (size_t)lrow * C::RSTRIDE, t, tws, none_load,
-                                                        none_store);
+        fft::transform_row_tws<N, C::TPR, false, false, true>(fsm + (size_t)lrow * C::RSTRIDE, t, tws,
+                                                              none_load, none_store);
+        __syncthreads();
         FengArgs a;
         Block8 b;
         unit(u, a, b);

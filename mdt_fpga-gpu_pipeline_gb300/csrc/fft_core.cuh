@@ -241,6 +241,24 @@ __device__ __forceinline__ void dft<16>(float2 *v)
     for (int k = 0; k < 16; k++) v[k] = y[k];
 }
 
+// Barrier between the phases of a pass: the block's, or with ROWSYNC the row's
+// (threadIdx.x / TPR).  Rows share nothing, so each then goes at its own pace and its
+// shared-memory phases overlap the others' arithmetic: a warp holds the row or whole
+// rows, or the row has a named barrier (1 + row).  It pays where one large block has
+// the SM (FP32 blocked F-engine, Nch 2048, 8 taps, 168 M samples: 1.50 -> 1.39 ms; bf16
+// 1.70 -> 1.61) and costs where the rows of small blocks should read memory
+// together (1024-point transforms of 38,912 rows: 114 -> 145 us).
+template <int TPR, bool ROWSYNC>
+__device__ __forceinline__ void pass_sync()
+{
+    if constexpr (!ROWSYNC)
+        __syncthreads();
+    else if constexpr (TPR <= 32)
+        __syncwarp();
+    else
+        asm volatile("bar.sync %0, %1;" ::"r"((int)threadIdx.x / TPR + 1), "n"(TPR) : "memory");
+}
+
 // One Stockham pass over one row.  `t` is the thread's index within the row
 // (0..TPR-1); every thread of the block must call every pass (barriers).
 // LOADFN (pass 0 only): inputs come from load(i) instead of shared memory,
@@ -250,7 +268,7 @@ __device__ __forceinline__ void dft<16>(float2 *v)
 // strides are multiples of 16 (pad(x + 16k) = pad(x) + 17k).
 // TWS: twiddles from the compact table `tws` (shared memory) instead of the
 //   device table `tw`.
-template <int N, int TPR, int P, bool LOADFN, bool STOREFN, bool TWS, class Load, class Store>
+template <int N, int TPR, int P, bool LOADFN, bool STOREFN, bool TWS, bool ROWSYNC, class Load, class Store>
 __device__ __forceinline__ void stockham_pass(float2 *sx, int t,
                                               const float2 *__restrict__ tw, const float2 *tws,
                                               Load &load, Store &store)
@@ -326,7 +344,7 @@ __device__ __forceinline__ void stockham_pass(float2 *sx, int t,
             dft<R>(v[k]);
         }
     }
-    if constexpr (!LOADFN) __syncthreads();  // every read of this pass precedes any write
+    if constexpr (!LOADFN) pass_sync<TPR, ROWSYNC>();  // every read of this pass precedes any write
 #pragma unroll
     for (int k = 0; k < NBT; k++) {
         const int b = t + k * TPR;
@@ -344,18 +362,18 @@ __device__ __forceinline__ void stockham_pass(float2 *sx, int t,
             }
         }
     }
-    if constexpr (!STOREFN) __syncthreads();  // writes visible to the next pass
+    if constexpr (!STOREFN) pass_sync<TPR, ROWSYNC>();  // writes visible to the next pass
 }
 
-template <int N, int TPR, int P, bool LOADFN, bool STOREFN, bool TWS, class Load, class Store>
+template <int N, int TPR, int P, bool LOADFN, bool STOREFN, bool TWS, bool ROWSYNC, class Load, class Store>
 __device__ __forceinline__ void run_passes(float2 *sx, int t, const float2 *__restrict__ tw,
                                            const float2 *tws, Load &load, Store &store)
 {
     constexpr int NP = Shape<N>::NPASS;
-    stockham_pass<N, TPR, P, LOADFN && P == 0, STOREFN && P == NP - 1, TWS>(sx, t, tw, tws, load,
-                                                                             store);
+    stockham_pass<N, TPR, P, LOADFN && P == 0, STOREFN && P == NP - 1, TWS, ROWSYNC>(sx, t, tw, tws,
+                                                                                      load, store);
     if constexpr (P + 1 < NP)
-        run_passes<N, TPR, P + 1, LOADFN, STOREFN, TWS>(sx, t, tw, tws, load, store);
+        run_passes<N, TPR, P + 1, LOADFN, STOREFN, TWS, ROWSYNC>(sx, t, tw, tws, load, store);
 }
 
 // Transforms one row: first-pass inputs from load(i) (LOADFN) or from the
@@ -368,16 +386,18 @@ template <int N, int TPR, bool LOADFN, bool STOREFN, class Load, class Store>
 __device__ __forceinline__ void transform_row(float2 *sx, int t, const float2 *__restrict__ tw,
                                               Load &load, Store &store)
 {
-    run_passes<N, TPR, 0, LOADFN, STOREFN, false>(sx, t, tw, nullptr, load, store);
+    run_passes<N, TPR, 0, LOADFN, STOREFN, false, false>(sx, t, tw, nullptr, load, store);
 }
 
 // As transform_row, with the twiddles read from the compact table `tws`
-// (filled by fill_tw_compact<N> and synchronised before the call).
-template <int N, int TPR, bool LOADFN, bool STOREFN, class Load, class Store>
+// (filled by fill_tw_compact<N> and synchronised before the call).  With ROWSYNC the
+// row is threadIdx.x / TPR, blocks are whole warps, and other rows may still be in
+// their passes when it returns.
+template <int N, int TPR, bool LOADFN, bool STOREFN, bool ROWSYNC, class Load, class Store>
 __device__ __forceinline__ void transform_row_tws(float2 *sx, int t, const float2 *tws, Load &load,
                                                   Store &store)
 {
-    run_passes<N, TPR, 0, LOADFN, STOREFN, true>(sx, t, nullptr, tws, load, store);
+    run_passes<N, TPR, 0, LOADFN, STOREFN, true, ROWSYNC>(sx, t, nullptr, tws, load, store);
 }
 
 }  // namespace fft
