@@ -67,6 +67,22 @@ struct FengArgs {
     float2 *X;
 };
 
+// Two int8 (re, im) samples as packed pairs, without the conversion unit: byte
+// u = x + 128 placed in the mantissa of 2^23 gives 2^23 + u exactly, and subtracting
+// 2^23 + 128 leaves x exactly.
+__device__ __forceinline__ void iq_pair(uint32_t word, float2 &xr, float2 &xi)
+{
+    const uint32_t v = word ^ 0x80808080u;
+    constexpr float kOff = -8388736.0f;  // -(2^23 + 128)
+    const float2 off = make_float2(kOff, kOff);
+    xr = __fadd2_rn(make_float2(__uint_as_float(__byte_perm(v, 0x4B000000u, 0x7540)),
+                                __uint_as_float(__byte_perm(v, 0x4B000000u, 0x7542))),
+                    off);
+    xi = __fadd2_rn(make_float2(__uint_as_float(__byte_perm(v, 0x4B000000u, 0x7541)),
+                                __uint_as_float(__byte_perm(v, 0x4B000000u, 0x7543))),
+                    off);
+}
+
 // Polyphase tap sum of the block's rows into shared memory (natural channel
 // order, padded): each work item is 8 consecutive channels of one row, read
 // as one 16-byte int8 I/Q vector and two float4 window vectors per tap;
@@ -79,38 +95,46 @@ __device__ __forceinline__ void pfb_rows_to_smem(const FengArgs &a, long row0, i
 {
     constexpr int ITEMS = ROWS * (N / 8);
     const long rows = (long)a.nsp * a.ne, hrows = (long)a.nhist * a.ne;
+    const long rowlen = (long)a.ne * N;
     for (int it = threadIdx.x; it < ITEMS; it += THREADS) {
         const int r = it / (N / 8);
         const int c0 = (it - r * (N / 8)) * 8;
         const long row = row0 + (long)r * step;
-        float re[8], im[8];
+        float2 re[4], im[4];  // of the channel pairs
 #pragma unroll
-        for (int k = 0; k < 8; k++) re[k] = im[k] = 0.0f;
+        for (int k = 0; k < 4; k++) re[k] = im[k] = make_float2(0.f, 0.f);
         if (row < rows) {
-            for (int i = 0; i < a.ntaps; i++) {
-                const long in = row + (long)i * a.ne;
-                const char2 *src = in < hrows ? a.hist + in * N : a.iq + (in - hrows) * N;
-                const int4 raw = __ldg(reinterpret_cast<const int4 *>(src + c0));
-                const float4 w0 = __ldg(reinterpret_cast<const float4 *>(a.win + (long)i * N + c0));
-                const float4 w1 =
-                    __ldg(reinterpret_cast<const float4 *>(a.win + (long)i * N + c0 + 4));
-                const float w[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
-                const int words[4] = {raw.x, raw.y, raw.z, raw.w};
+            const float *win = a.win + c0;
+            auto taps = [&](const char2 *src, int n) {
+#pragma unroll 4
+                for (int i = 0; i < n; i++, src += rowlen, win += N) {
+                    const int4 raw = __ldg(reinterpret_cast<const int4 *>(src));
+                    const float4 w0 = __ldg(reinterpret_cast<const float4 *>(win));
+                    const float4 w1 = __ldg(reinterpret_cast<const float4 *>(win + 4));
+                    const float2 w[4] = {make_float2(w0.x, w0.y), make_float2(w0.z, w0.w),
+                                         make_float2(w1.x, w1.y), make_float2(w1.z, w1.w)};
+                    const int words[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
-                for (int k = 0; k < 8; k++) {
-                    const int word = words[k >> 1];
-                    const int sh = (k & 1) * 16;
-                    const float xr = (float)(signed char)((word >> sh) & 0xff);
-                    const float xi = (float)(signed char)((word >> (sh + 8)) & 0xff);
-                    re[k] = __fmaf_rn(w[k], xr, re[k]);
-                    im[k] = __fmaf_rn(w[k], xi, im[k]);
+                    for (int k = 0; k < 4; k++) {
+                        float2 xr, xi;
+                        iq_pair((uint32_t)words[k], xr, xi);
+                        re[k] = __ffma2_rn(w[k], xr, re[k]);
+                        im[k] = __ffma2_rn(w[k], xi, im[k]);
+                    }
                 }
-            }
+            };
+            // the taps on the history, then those on this call's input
+            const int nh = row < hrows ? (int)min((long)a.ntaps, (hrows - row + a.ne - 1) / a.ne) : 0;
+            if (nh > 0) taps(a.hist + row * N + c0, nh);
+            taps(a.iq + (row + (long)nh * a.ne - hrows) * N + c0, a.ntaps - nh);
         }
         float2 *sx = smem + (size_t)r * rstride;
         const int p0 = fft::pad(c0);  // c0 % 8 == 0: pad(c0 + k) = p0 + k for k < 8
 #pragma unroll
-        for (int k = 0; k < 8; k++) sx[p0 + k] = make_float2(re[k], im[k]);
+        for (int k = 0; k < 4; k++) {
+            sx[p0 + 2 * k] = make_float2(re[k].x, im[k].x);
+            sx[p0 + 2 * k + 1] = make_float2(re[k].y, im[k].y);
+        }
     }
 }
 
@@ -147,8 +171,10 @@ __global__ void __launch_bounds__(FengCfg<N, R>::THREADS, FengCfg<N, R>::MINB)
 // registers and converts each input spectrum from int8 once: input spectrum
 // s0+j feeds row r at tap j-r, and the unrolled loop over j visits every
 // row's taps in increasing order, so each output is the same fmaf chain as
-// PpS_Batch (bit-identical).  NT is Ntaps as a compile-time constant (4 or
-// 8); other tap counts use the per-row tap sum above.  Consecutive blocks
+// PpS_Batch (bit-identical).  NT is Ntaps as a compile-time constant (4, 8
+// or, from 256 channels on, 16: 20,000 rows of Nch 2048 FP32 355 us, by the per-row
+// sum 470; of Nch 128 the per-row sum is the faster, 386 and 485 for 400,000); other
+// tap counts use the per-row tap sum above.  Consecutive blocks
 // are the four 8-spectrum groups of one (element, 32-spectrum chunk), so
 // their inputs overlap in L2 and their partial output rows meet there.
 
@@ -162,12 +188,6 @@ constexpr int SB8 = 8;  // spectra per block
 // Channels from which the spectrum-block kernels run as persistent blocks.
 #ifndef MDT_FENG_PERSIST
 #define MDT_FENG_PERSIST 512
-#endif
-
-// Tap sums of the spectrum-block kernels convert int8 samples with integer
-// and FP32 add instructions instead of the int-to-float conversion unit.
-#ifndef MDT_FENG_I2F_MAGIC
-#define MDT_FENG_I2F_MAGIC 1
 #endif
 
 template <int N>
@@ -186,45 +206,6 @@ struct FengBCfg {
     static constexpr size_t STAGE_OFF = (sizeof(float2) * (size_t)RSTRIDE * SB8 + 15) / 16 * 16;
     static constexpr size_t TW_OFF = STAGE_OFF + (size_t)(SB8 + 7) * 2 * N;
     static constexpr size_t SMEM = TW_OFF + sizeof(float2) * (size_t)fft::tw_compact_len<N>();
-};
-
-template <int CPI>
-struct Samples;
-template <>
-struct Samples<1> {
-    float re[1], im[1];
-    __device__ __forceinline__ void load_shared(const uint8_t *p)
-    {
-        const char2 v = *reinterpret_cast<const char2 *>(p);
-        re[0] = (float)v.x;
-        im[0] = (float)v.y;
-    }
-    __device__ __forceinline__ void load(const char2 *p, bool ok)
-    {
-        const char2 v = ok ? __ldg(p) : make_char2(0, 0);
-        re[0] = (float)v.x;
-        im[0] = (float)v.y;
-    }
-};
-template <>
-struct Samples<2> {
-    float re[2], im[2];
-    __device__ __forceinline__ void load_shared(const uint8_t *p)
-    {
-        const char4 v = *reinterpret_cast<const char4 *>(p);
-        re[0] = (float)v.x;
-        im[0] = (float)v.y;
-        re[1] = (float)v.z;
-        im[1] = (float)v.w;
-    }
-    __device__ __forceinline__ void load(const char2 *p, bool ok)
-    {
-        const char4 v = ok ? __ldg(reinterpret_cast<const char4 *>(p)) : make_char4(0, 0, 0, 0);
-        re[0] = (float)v.x;
-        im[0] = (float)v.y;
-        re[1] = (float)v.z;
-        im[1] = (float)v.w;
-    }
 };
 
 // 16-byte asynchronous global->shared copy; src_bytes 0 fills zeros.
@@ -260,102 +241,81 @@ __device__ __forceinline__ void stage_rows_async(const FengArgs &a, int s0, int 
     asm volatile("cp.async.commit_group;" ::: "memory");
 }
 
-// Waits for the staged rows, then forms the block's 8 tap sums from them
-// into the transform rows (no barrier after the sums).
+// The block's 8 tap sums into the transform rows.  fetch(j, c) reads the samples
+// of channels c and c + 1 of input spectrum s0 + j; the two channels are one packed
+// FP32 pair: one f32x2 fma per (row, tap) and component, each lane rounded as fmaf.
+// With more than 8 taps a window value is loaded for the first spectrum that meets it
+// (it serves eight).
+template <int N, int NT, int THREADS, class Fetch>
+__device__ __forceinline__ void tap_sums(const FengArgs &a, int s0, float2 *smem, int rstride,
+                                         Fetch &&fetch)
+{
+    // rows of an item: all 8, or 4 where the block has more threads than channel pairs
+    constexpr int RPI = N / 2 < THREADS ? SB8 / 2 : SB8;
+    for (int it = threadIdx.x; it < N / 2 * (SB8 / RPI); it += THREADS) {
+        const int c0 = 2 * (it % (N / 2)), r0 = it / (N / 2) * RPI;
+        const float2 *win = reinterpret_cast<const float2 *>(a.win + c0);
+        float2 w2[NT];
+        if constexpr (NT <= 8) {
+#pragma unroll
+            for (int i = 0; i < NT; i++) w2[i] = __ldg(win + (long)i * (N / 2));
+        }
+        float2 ar[RPI], ai[RPI];
+#pragma unroll
+        for (int r = 0; r < RPI; r++) ar[r] = ai[r] = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int j = 0; j < RPI + NT - 1; j++) {
+            if constexpr (NT > 8) {
+                if (j < NT) w2[j] = __ldg(win + (long)j * (N / 2));
+            }
+            float2 xr, xi;
+            iq_pair(fetch(r0 + j, c0), xr, xi);
+#pragma unroll
+            for (int r = 0; r < RPI; r++) {
+                const int i = j - r;
+                if (i >= 0 && i < NT) {
+                    ar[r] = __ffma2_rn(w2[i], xr, ar[r]);
+                    ai[r] = __ffma2_rn(w2[i], xi, ai[r]);
+                }
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < RPI; r++) {
+            const bool live = s0 + r0 + r < a.nsp;
+            float2 *row = smem + (size_t)(r0 + r) * rstride + fft::pad(c0);  // pad(c0 + 1) = pad(c0) + 1
+            row[0] = live ? make_float2(ar[r].x, ai[r].x) : make_float2(0.f, 0.f);
+            row[1] = live ? make_float2(ar[r].y, ai[r].y) : make_float2(0.f, 0.f);
+        }
+    }
+}
+
+// Waits for the staged rows, then forms the block's 8 tap sums from them (no barrier
+// after the sums).
 template <int N, int NT, int THREADS>
 __device__ __forceinline__ void tapsum_from_stage(const FengArgs &a, int s0, float2 *smem, int rstride,
                                                   const uint8_t *stage)
 {
-    constexpr int CPI = (N / THREADS >= 2) ? 2 : 1;  // channels per thread item
-    constexpr int ITEMS = N / CPI;
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
-    for (int it = threadIdx.x; it < ITEMS; it += THREADS) {
-        const int c0 = it * CPI;
-        if constexpr (CPI == 2 && MDT_FFT_F32X2) {
-            // the two channels c0, c0 + 1 as one packed FP32 pair: one f32x2
-            // fma per (row, tap) and component, each lane rounded as fmaf
-            float2 w2[NT];
-#pragma unroll
-            for (int i = 0; i < NT; i++)
-                w2[i] = __ldg(reinterpret_cast<const float2 *>(a.win + (long)i * N + c0));
-            float2 ar[SB8], ai[SB8];
-#pragma unroll
-            for (int r = 0; r < SB8; r++) ar[r] = ai[r] = make_float2(0.f, 0.f);
-#pragma unroll
-            for (int j = 0; j < SB8 + NT - 1; j++) {
-#if MDT_FENG_I2F_MAGIC
-                // int8 -> float without the conversion unit: byte u = x + 128
-                // placed in the mantissa of 2^23 gives 2^23 + u exactly, and
-                // subtracting 2^23 + 128 leaves x exactly
-                const uint32_t wv =
-                    *reinterpret_cast<const uint32_t *>(stage + (size_t)j * 2 * N + 2 * c0) ^ 0x80808080u;
-                constexpr float kOff = -8388736.0f;  // -(2^23 + 128)
-                const float2 off = make_float2(kOff, kOff);
-                const float2 xr = __fadd2_rn(make_float2(__uint_as_float(__byte_perm(wv, 0x4B000000u, 0x7540)),
-                                                         __uint_as_float(__byte_perm(wv, 0x4B000000u, 0x7542))),
-                                             off);
-                const float2 xi = __fadd2_rn(make_float2(__uint_as_float(__byte_perm(wv, 0x4B000000u, 0x7541)),
-                                                         __uint_as_float(__byte_perm(wv, 0x4B000000u, 0x7543))),
-                                             off);
-#else
-                Samples<2> x;
-                x.load_shared(stage + (size_t)j * 2 * N + 2 * c0);
-                const float2 xr = make_float2(x.re[0], x.re[1]), xi = make_float2(x.im[0], x.im[1]);
-#endif
-#pragma unroll
-                for (int r = 0; r < SB8; r++) {
-                    const int i = j - r;
-                    if (i >= 0 && i < NT) {
-                        ar[r] = __ffma2_rn(w2[i], xr, ar[r]);
-                        ai[r] = __ffma2_rn(w2[i], xi, ai[r]);
-                    }
-                }
-            }
-#pragma unroll
-            for (int r = 0; r < SB8; r++) {
-                const bool live = s0 + r < a.nsp;
-                float2 *row = smem + (size_t)r * rstride + fft::pad(c0);  // pad(c0 + 1) = pad(c0) + 1
-                row[0] = live ? make_float2(ar[r].x, ai[r].x) : make_float2(0.f, 0.f);
-                row[1] = live ? make_float2(ar[r].y, ai[r].y) : make_float2(0.f, 0.f);
-            }
-            continue;
-        }
-        float w[NT][CPI];
-#pragma unroll
-        for (int i = 0; i < NT; i++)
-#pragma unroll
-            for (int k = 0; k < CPI; k++) w[i][k] = __ldg(a.win + (long)i * N + c0 + k);
-        float ar[SB8][CPI], ai[SB8][CPI];
-#pragma unroll
-        for (int r = 0; r < SB8; r++)
-#pragma unroll
-            for (int k = 0; k < CPI; k++) ar[r][k] = ai[r][k] = 0.0f;
-#pragma unroll
-        for (int j = 0; j < SB8 + NT - 1; j++) {
-            Samples<CPI> x;
-            x.load_shared(stage + (size_t)j * 2 * N + 2 * c0);
-#pragma unroll
-            for (int r = 0; r < SB8; r++) {
-                const int i = j - r;
-                if (i >= 0 && i < NT) {
-#pragma unroll
-                    for (int k = 0; k < CPI; k++) {
-                        ar[r][k] = __fmaf_rn(w[i][k], x.re[k], ar[r][k]);
-                        ai[r][k] = __fmaf_rn(w[i][k], x.im[k], ai[r][k]);
-                    }
-                }
-            }
-        }
-#pragma unroll
-        for (int r = 0; r < SB8; r++) {
-            const bool live = s0 + r < a.nsp;
-#pragma unroll
-            for (int k = 0; k < CPI; k++)
-                smem[(size_t)r * rstride + fft::pad(c0 + k)] =
-                    live ? make_float2(ar[r][k], ai[r][k]) : make_float2(0.f, 0.f);
-        }
-    }
+    tap_sums<N, NT, THREADS>(a, s0, smem, rstride, [&](int j, int c) -> uint32_t {
+        return *reinterpret_cast<const uint32_t *>(stage + (size_t)j * 2 * N + 2 * c);
+    });
+}
+
+// The same from global memory.
+template <int N, int NT, int THREADS>
+__device__ __forceinline__ void tapsum_from_global(const FengArgs &a, int s0, int e, float2 *smem,
+                                                   int rstride)
+{
+    const long rowlen = (long)a.ne * N;
+    const int nin = a.nsp + NT - 1;  // input spectra of this integration
+    tap_sums<N, NT, THREADS>(a, s0, smem, rstride, [&](int j, int c) -> uint32_t {
+        const int sp = s0 + j;
+        if (sp >= nin) return 0u;
+        const char2 *p = (sp < a.nhist ? a.hist + (long)sp * rowlen
+                                       : a.iq + (long)(sp - a.nhist) * rowlen) + (long)e * N + c;
+        return __ldg(reinterpret_cast<const uint32_t *>(p));
+    });
 }
 
 // Stage, then tap sum; `mid()` runs while the copies are in flight.
@@ -393,7 +353,10 @@ __device__ __forceinline__ void fengine_block8(const FengArgs &a, const Block8 &
     using C = FengBCfg<N>;
     float2 *tws = reinterpret_cast<float2 *>(reinterpret_cast<uint8_t *>(fsm) + C::TW_OFF);
     auto fill_tw = [&]() { fft::fill_tw_compact<N>(tws, a.tw, (int)threadIdx.x, C::THREADS); };
-    if constexpr (NT > 0) {
+    if constexpr (NT > 8) {
+        fill_tw();
+        tapsum_from_global<N, NT, C::THREADS>(a, b.s0, b.e, fsm, C::RSTRIDE);
+    } else if constexpr (NT > 0) {
         pfb_block8_to_smem<N, NT, C::THREADS>(a, b.s0, b.e, fsm, C::RSTRIDE,
                                               reinterpret_cast<uint8_t *>(fsm) + C::STAGE_OFF,
                                               fill_tw);
@@ -495,7 +458,7 @@ __device__ __forceinline__ void fengine_units(int u, int step, int nunits, const
 template <int N, int NT>
 constexpr bool feng_persistent()
 {
-    return NT > 0 && N >= MDT_FENG_PERSIST;
+    return (NT == 4 || NT == 8) && N >= MDT_FENG_PERSIST;
 }
 
 // Blocks of a spectrum-block launch over `units`.
@@ -715,8 +678,10 @@ static mdt_status dispatch_block8(int nch, int ntaps, F f)
 {
 #define MDT_NT_CASES(NV)                                                       \
     case NV:                                                                   \
-        return ntaps == 4 ? f.template run<NV, 4>()                            \
-                          : (ntaps == 8 ? f.template run<NV, 8>() : f.template run<NV, 0>());
+        return ntaps == 4    ? f.template run<NV, 4>()                         \
+               : ntaps == 8  ? f.template run<NV, 8>()                         \
+               : ntaps == 16 ? f.template run<NV, (NV < 256 ? 0 : 16)>()       \
+                             : f.template run<NV, 0>();
     switch (nch) {
         MDT_NT_CASES(32)
         MDT_NT_CASES(64)
@@ -828,7 +793,7 @@ struct FengBatchRun {
     template <int N, int NT>
     mdt_status run()
     {
-        if constexpr (NT == 0) {
+        if constexpr (NT != 4 && NT != 8) {
             return invalid("batched F-engine: Ntaps must be 4 or 8");
         } else {
             using C = FengBCfg<N>;

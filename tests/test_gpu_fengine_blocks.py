@@ -12,7 +12,8 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("nch", [128, 256, 512, 1024, 2048])
-@pytest.mark.parametrize("ntaps,ne,nsp", [(4, 37, 250), (8, 37, 250), (8, 3, 9), (5, 11, 70)])
+@pytest.mark.parametrize("ntaps,ne,nsp", [(4, 37, 250), (8, 37, 250), (8, 3, 9), (5, 11, 70),
+                                           (16, 37, 250), (16, 5, 11)])
 def test_blocks_match_rows(mdt, cuda, nch, ntaps, ne, nsp):
     g = torch.Generator(device="cuda")
     g.manual_seed(nch + 7 * ntaps + nsp)
