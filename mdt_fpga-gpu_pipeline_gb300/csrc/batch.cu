@@ -365,7 +365,7 @@ MDT_API mdt_status mdt_fx_batch_create(const mdt_fx_desc *descs, int njobs, mdt_
         f.blk0 = (int)g.nblocks;
         f.wk0 = (int)g.nwork;
         g.nblocks += mdt::fjob_blocks(d.nelements, b->nkc[j]);
-        g.nwork += mdt::fjob_tc_items(d.nelements, d.nspectra);
+        g.nwork += mdt::fjob_tc_groups(d.nelements, d.nspectra);
         g.count++;
         b->h_fjobs.push_back(f);
         b->fjob_of.push_back(j);

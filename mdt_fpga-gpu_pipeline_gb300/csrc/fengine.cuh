@@ -13,11 +13,11 @@ struct FJob {
     int ne, nsp, nep, nkc;
     float scale;
     int blk0;          // first block of the job (prefix sum over the launch)
-    int wk0;           // first work item of the job in a tensor-core F-engine launch
+    int wk0;           // first group of the job in a tensor-core F-engine launch
 };
 
-// Work items of one job in a tensor-core F-engine launch (runs of 512 spectra).
-inline long fjob_tc_items(int ne, int nsp) { return (long)ne * ((nsp + 511) / 512); }
+// Groups (32 spectra of one element) of one job in a tensor-core F-engine launch.
+inline long fjob_tc_groups(int ne, int nsp) { return (long)ne * ((nsp + 31) / 32); }
 // Whether the tensor-core F-engine handles this shape.
 inline bool fengine_tc_shape(int nch, int ntaps) { return nch == 1024 && (ntaps == 4 || ntaps == 8); }
 
@@ -28,7 +28,7 @@ mdt_status fengine_x16_batched(int nch, int ntaps, const FJob *jobs, int njobs, 
                                cudaStream_t stream);
 // Batched tensor-core F-engine (f16 output) over jobs of Nch 1024 and one
 // Ntaps (4 or 8); `jobs` is a device array with wk0 prefix sums, `nwork` the
-// total work items.
+// total groups.
 mdt_status fengine_tc_batched(int ntaps, const FJob *jobs, int njobs, long nwork, int *err,
                               cudaStream_t stream);
 // The FP32 path's F-output XB: complex64 in blocks of 8 spectra (ceil(Nsp/8)

@@ -44,7 +44,7 @@ constexpr int NSLOT = 4;                // input ring slots
 constexpr int US = 8;                   // spectra per unit
 constexpr int CPT = N / PT;             // channels per PFB thread
 constexpr int ROWB = 2 * N;             // one (spectrum, element) row of int8 I/Q
-constexpr int RUN = 512;                // spectra per work item
+constexpr int GS = 32;                  // spectra of a group, the unit in which work is split
 constexpr uint32_t TILE = 16384;        // 128 rows x 128 bytes
 // shared memory: the 128 x 128 block-diagonal DFT operand of MMA 2 as two
 // 128-row tiles of K 64 (the first 64 rows of the first tile are MMA 1's
@@ -85,7 +85,7 @@ __host__ __device__ constexpr uint32_t bar_count(int b)
 }
 
 // One launch: a single job (with optional PFB history) or a device table of
-// jobs (FJob, work items from wk0).
+// jobs (FJob, groups from wk0).
 struct Launch {
     FJob one;
     const char2 *hist;  // first nhist spectra of the single job (may be null)
@@ -240,11 +240,20 @@ __device__ __forceinline__ bool wait_or_abort(uint32_t bar, uint32_t parity, vol
     return true;
 }
 
-// Work item w of the launch -> job (updates `a` / `cur`), element, first
-// spectrum, number of 8-spectrum units.
+// The groups (32 spectra of one element; a job's are element by element from wk0 on)
+// are split evenly: CTA b takes [first_group(b), first_group(b + 1)).  A work item is
+// the CTA's part of one element: each has a lead-in of Ntaps - 1 rows, so whole
+// stretches cost least.  f16, 8 taps: NE=256, Nsp=4096 1.88 ms, with items of 512 spectra
+// dealt in turn 1.95 (14 rounds where 13.5 would do); NE=40, Nsp=1000, 80 such items for
+// 152 SMs, 98 us and 154.
 struct Item {
-    int e, s0, nunits;
+    int e, s0, nunits, ngroups;
 };
+__device__ __forceinline__ int first_group(const Launch &L, int b)
+{
+    return (int)((long)L.nwork * b / gridDim.x);
+}
+// The job of group w (updates `a` / `cur`; true if it changed).
 __device__ __forceinline__ bool next_job(const Launch &L, int w, FJob &a, int &cur)
 {
     int j = cur < 0 ? 0 : cur;
@@ -255,14 +264,17 @@ __device__ __forceinline__ bool next_job(const Launch &L, int w, FJob &a, int &c
     cur = j;
     return true;
 }
-__device__ __forceinline__ Item item_of(const FJob &a, int w)
+// The work item from group w on, of the CTA's groups up to w1.
+__device__ __forceinline__ Item item_of(const FJob &a, int w, int w1)
 {
-    const int runs_per_e = (a.nsp + RUN - 1) / RUN;
+    const int per_e = (a.nsp + GS - 1) / GS;
     const int wl = w - a.wk0;
     Item it;
-    it.e = wl / runs_per_e;
-    it.s0 = (wl % runs_per_e) * RUN;
-    it.nunits = (min(it.s0 + RUN, a.nsp) - it.s0 + US - 1) / US;
+    it.e = wl / per_e;
+    const int k = wl - it.e * per_e;
+    it.ngroups = min(per_e - k, w1 - w);
+    it.s0 = k * GS;
+    it.nunits = (min(it.s0 + it.ngroups * GS, a.nsp) - it.s0 + US - 1) / US;
     return it;
 }
 
@@ -356,6 +368,7 @@ __global__ void __launch_bounds__(THREADS, 1) fengine_tc_kernel(Launch L)
         return __all_sync(0xffffffffu, okw);
     };
     const uint32_t gR = sbase + OFF_RING;
+    const int w0 = first_group(L, blockIdx.x), w1 = first_group(L, blockIdx.x + 1);
 
     if (tid < PT) {
         // ============================================================ PFB role
@@ -369,7 +382,7 @@ __global__ void __launch_bounds__(THREADS, 1) fengine_tc_kernel(Launch L)
         long n = 0, r = 0;  // units and ring uses of this CTA so far
         FJob a = L.one;
         int cur = -1;
-        for (int w = blockIdx.x; w < L.nwork && ok; w += gridDim.x) {
+        for (int w = w0; w < w1 && ok;) {
             if (next_job(L, w, a, cur)) {
                 // the job's scaled window for this thread's own channels (only this thread reads them)
 #pragma unroll
@@ -383,8 +396,9 @@ __global__ void __launch_bounds__(THREADS, 1) fengine_tc_kernel(Launch L)
                                                             __ldg(a.win + (2 * pr + 1) * N + c) * a.scale);
                 }
             }
-            const Item it = item_of(a, w);
+            const Item it = item_of(a, w, w1);
             const int nunits = it.nunits;
+            w += it.ngroups;
             {  // ---- lead-in use: the item's first Ntaps-1 rows into the carry
                 const int slot = (int)(r % NSLOT);
                 if (!wait_warp(bar(BAR_FULL + slot), (uint32_t)((r / NSLOT) & 1))) {
@@ -575,9 +589,10 @@ __global__ void __launch_bounds__(THREADS, 1) fengine_tc_kernel(Launch L)
             }
             return true;
         };
-        for (int w = blockIdx.x; w < L.nwork && ok; w += gridDim.x) {
+        for (int w = w0; w < w1 && ok;) {
             next_job(L, w, a, cur);
-            const Item it = item_of(a, w);
+            const Item it = item_of(a, w, w1);
+            w += it.ngroups;
             const int e = it.e, s0 = it.s0, nunits = it.nunits;
             for (int u = 0; u < nunits; u++, n++) {
                 const int b = (int)(n & 1);
@@ -630,13 +645,15 @@ __global__ void __launch_bounds__(THREADS, 1) fengine_tc_kernel(Launch L)
         {
             FJob a2 = L.one;
             int c2 = -1;
-            for (int w = blockIdx.x; w < L.nwork; w += gridDim.x) {
+            for (int w = w0; w < w1;) {
                 next_job(L, w, a2, c2);
-                total_uses += 1 + item_of(a2, w).nunits;
+                const Item it = item_of(a2, w, w1);
+                w += it.ngroups;
+                total_uses += 1 + it.nunits;
             }
         }
         FJob al = L.one;
-        int curl = -1, wl = blockIdx.x, ul = -1;  // ul = -1: the item's lead-in use
+        int curl = -1, wl = w0, ul = -1;  // ul = -1: the item's lead-in use
         Item itl{};
         const int nhist = L.table ? 0 : L.nhist;
         auto row_src = [&](long rho, int e) -> const char2 * {
@@ -654,7 +671,7 @@ __global__ void __launch_bounds__(THREADS, 1) fengine_tc_kernel(Launch L)
             }
             if (ul < 0) {
                 next_job(L, wl, al, curl);
-                itl = item_of(al, wl);
+                itl = item_of(al, wl, w1);
             }
             long r0;
             int cnt;
@@ -673,7 +690,7 @@ __global__ void __launch_bounds__(THREADS, 1) fengine_tc_kernel(Launch L)
                 tc::bulk_g2s(dst + (uint32_t)(q * ROWB), row_src(r0 + q, itl.e), ROWB, full);
             if (++ul == itl.nunits) {
                 ul = -1;
-                wl += gridDim.x;
+                wl += itl.ngroups;
             }
         }
         // the copies issued are complete before the CTA ends (bounded waits)
@@ -689,9 +706,11 @@ __global__ void __launch_bounds__(THREADS, 1) fengine_tc_kernel(Launch L)
         {
             FJob a2 = L.one;
             int c2 = -1;
-            for (int w = blockIdx.x; w < L.nwork; w += gridDim.x) {
+            for (int w = w0; w < w1;) {
                 next_job(L, w, a2, c2);
-                total_units += item_of(a2, w).nunits;
+                const Item it = item_of(a2, w, w1);
+                w += it.ngroups;
+                total_units += it.nunits;
             }
         }
         // MMA 1 of unit u: accumulator buffer u % 2 <- P tiles x DFT
@@ -808,7 +827,7 @@ mdt_status fengine_tc(int ne, int nch, int ntaps, int nsp, const int8_t *hist, i
         return invalid("fengine_tc: bad arguments");
     if (((uintptr_t)iq | (uintptr_t)hist | (uintptr_t)X16) & 15)
         return invalid("fengine_tc: buffers must be 16-byte aligned");
-    const long nwork = fjob_tc_items(ne, nsp);
+    const long nwork = fjob_tc_groups(ne, nsp);
     if (nwork > 0x7fffffffL) return invalid("fengine_tc: too many work items");
     ftc::Launch L{};
     L.one.iq = reinterpret_cast<const char2 *>(iq);
