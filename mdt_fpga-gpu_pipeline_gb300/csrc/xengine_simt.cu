@@ -92,6 +92,11 @@ __device__ __forceinline__ int xs_off(int e, int kk)
     return e * XS_ROWB + ((((kk >> 1) ^ ((e >> 2) & 7))) << 4) + ((kk & 1) << 3);
 }
 
+// SMALL: few micro-tiles (two channels of up to 28 elements) in four to sixteen K
+// slices each.  Their sums are added by one thread per value instead of one per
+// micro-tile, and fewer rows are staged: NE=10, Nch=1024, Nsp=64 8.3 us, 15.5 without;
+// NE=28, Nsp=16 13.4 and 14.8.  With fewer slices it costs (NE=38, Nsp=64: 31 us, 26).
+template <bool SMALL>
 __global__ void __launch_bounds__(XS_THREADS, 3) xengine_herm_f32_kernel(XengArgs a)
 {
     // [stage][operand][k][element]; the K-slice reduction reuses the space
@@ -129,8 +134,9 @@ __global__ void __launch_bounds__(XS_THREADS, 3) xengine_herm_f32_kernel(XengArg
     const float2 *Xc = a.Xptrs ? a.Xptrs[ch] : a.X + (long)ch * a.xstride;
     const float2 *Xc2 = !has2 ? Xc : (a.Xptrs ? a.Xptrs[ch + 1] : a.X + (long)(ch + 1) * a.xstride);
 
-    // stage chunk k0 into buffer st: 64 element rows of XS_KC samples per operand
+    // stage chunk k0 into buffer st: up to 64 element rows of XS_KC samples per operand
     auto stage = [&](int k0, int st) {
+        const int lgst = !SMALL ? 6 : nr <= 16 ? 4 : 5;  // the loops run over 16, 32 or 64 rows
         uint8_t *A = tileA(st), *B = tileB(st);
         // rows the micro-tiles read: rows past the operand's last element up to
         // the micro-tile edge are zero-filled, rows beyond it are not staged
@@ -138,8 +144,8 @@ __global__ void __launch_bounds__(XS_THREADS, 3) xengine_herm_f32_kernel(XengArg
             // blocks of 8 samples ld apart: every (8-sample block, element) is 64
             // contiguous bytes, copied as four 16-byte pairs; blocks past the input
             // are zero-filled
-            for (int idx = tid; idx < (XS_KC / 8) * XS_ST * 4; idx += XS_THREADS) {
-                const int q = idx & 3, e = (idx >> 2) & (XS_ST - 1), sbl = idx >> 8;
+            for (int idx = tid; idx < (XS_KC / 8 * 4) << lgst; idx += XS_THREADS) {
+                const int q = idx & 3, e = (idx >> 2) & ((1 << lgst) - 1), sbl = idx >> (lgst + 2);
                 const int kk = 8 * sbl + 2 * q;
                 const bool kin = k0 + 8 * sbl < a.nsp;
                 const long off = (long)((k0 >> 3) + sbl) * a.ld + 2 * q;
@@ -157,8 +163,8 @@ __global__ void __launch_bounds__(XS_THREADS, 3) xengine_herm_f32_kernel(XengArg
             }
         } else {
             // X[k*ld + e]: consecutive threads take consecutive elements of one sample
-            for (int idx = tid; idx < XS_KC * XS_ST; idx += XS_THREADS) {
-                const int kk = idx / XS_ST, e = idx - kk * XS_ST;
+            for (int idx = tid; idx < XS_KC << lgst; idx += XS_THREADS) {
+                const int kk = idx >> lgst, e = idx & ((1 << lgst) - 1);
                 const long off = (long)(k0 + kk) * a.ld;
                 const bool kin = k0 + kk < a.nsp;
                 const int dst = xs_off(e, kk);
@@ -253,9 +259,61 @@ __global__ void __launch_bounds__(XS_THREADS, 3) xengine_herm_f32_kernel(XengArg
         __syncthreads();  // buffer st is overwritten by the next stage() call
     }
 
-    // reduce the K slices in a fixed order (slice 0 + 1 + 2 ...)
+    auto channel = [&](int c) { return a.Vptrs ? a.Vptrs[c] : a.V + (long)c * a.vstride; };
+    // V[r, q] and its mirror from the sum v over the samples (r >= q)
+    auto output = [&](float2 *Vc, int r, int q, float2 v) {
+        if (r >= a.ne || q >= a.ne || r < q) return;
+        if (r == q) v.y = 0.f;  // autocorrelations are real
+        // lower:  V[r,q] = alpha v + beta V[r,q]
+        float2 lo = make_float2(a.alpha.x * v.x - a.alpha.y * v.y,
+                                a.alpha.x * v.y + a.alpha.y * v.x);
+        const long il = (long)q * a.ldv + r;
+        if (!a.beta_zero) {
+            const float2 o = Vc[il];
+            lo.x += a.beta.x * o.x - a.beta.y * o.y;
+            lo.y += a.beta.x * o.y + a.beta.y * o.x;
+        }
+        Vc[il] = lo;
+        if (r != q) {
+            // upper mirror: V[q,r] = alpha conj(v) + beta V[q,r]
+            float2 up = make_float2(a.alpha.x * v.x + a.alpha.y * v.y,
+                                    -a.alpha.x * v.y + a.alpha.y * v.x);
+            const long iu = (long)r * a.ldv + q;
+            if (!a.beta_zero) {
+                const float2 o = Vc[iu];
+                up.x += a.beta.x * o.x - a.beta.y * o.y;
+                up.y += a.beta.x * o.y + a.beta.y * o.x;
+            }
+            Vc[iu] = up;
+        }
+    };
+
+    // The K slices' sums through shared memory, added in a fixed order (slice 0 + 1 + 2 ...)
+    float2 *red = sbuf;  // ksl * nmt2 * 16 <= 256 * 16 complex
+    if constexpr (SMALL) {  // one value of one micro-tile per thread
+        if (active) {
+#pragma unroll
+            for (int i = 0; i < XS_MT; i++)
+#pragma unroll
+                for (int j = 0; j < XS_MT; j++) red[(ks * 16 + i * 4 + j) * nmt2 + mt2] = acc[i][j];
+        }
+        __syncthreads();
+        for (int idx = tid; idx < 16 * nmt2; idx += XS_THREADS) {
+            const int ij = idx / nmt2, m2 = idx - ij * nmt2, c2 = m2 / nmt, m = m2 - c2 * nmt;
+            if (c2 && !has2) continue;
+            int oi, oj;
+            pair_index(m, oi, oj);
+            float2 v = red[idx];
+            for (int s2 = 1; s2 < ksl; s2++) {
+                const float2 u = red[s2 * 16 * nmt2 + idx];
+                v.x += u.x;
+                v.y += u.y;
+            }
+            output(channel(ch + c2), r0 + oi * XS_MT + (ij >> 2), q0 + oj * XS_MT + (ij & 3), v);
+        }
+        return;
+    }
     if (ksl > 1) {
-        float2 *red = sbuf;  // (ksl-1)*nmt*16 < 256*16 complex
         if (active && ks > 0) {
 #pragma unroll
             for (int i = 0; i < XS_MT; i++)
@@ -277,41 +335,12 @@ __global__ void __launch_bounds__(XS_THREADS, 3) xengine_herm_f32_kernel(XengArg
         }
     }
     if (!active || ks != 0) return;
-
-    const int cho = ch + cs;  // output channel
-    float2 *Vc = a.Vptrs ? a.Vptrs[cho] : a.V + (long)cho * a.vstride;
+    float2 *Vc = channel(ch + cs);
 #pragma unroll
-    for (int i = 0; i < XS_MT; i++) {
+    for (int i = 0; i < XS_MT; i++)
 #pragma unroll
-        for (int j = 0; j < XS_MT; j++) {
-            const int r = r0 + mi * XS_MT + i, q = q0 + mj * XS_MT + j;
-            if (r >= a.ne || q >= a.ne || r < q) continue;
-            float2 v = acc[i][j];
-            if (r == q) v.y = 0.f;  // autocorrelations are real
-            // lower:  V[r,q] = alpha v + beta V[r,q]
-            float2 lo = make_float2(a.alpha.x * v.x - a.alpha.y * v.y,
-                                    a.alpha.x * v.y + a.alpha.y * v.x);
-            long il = (long)q * a.ldv + r;
-            if (!a.beta_zero) {
-                float2 o = Vc[il];
-                lo.x += a.beta.x * o.x - a.beta.y * o.y;
-                lo.y += a.beta.x * o.y + a.beta.y * o.x;
-            }
-            Vc[il] = lo;
-            if (r != q) {
-                // upper mirror: V[q,r] = alpha conj(v) + beta V[q,r]
-                float2 up = make_float2(a.alpha.x * v.x + a.alpha.y * v.y,
-                                        -a.alpha.x * v.y + a.alpha.y * v.x);
-                long iu = (long)r * a.ldv + q;
-                if (!a.beta_zero) {
-                    float2 o = Vc[iu];
-                    up.x += a.beta.x * o.x - a.beta.y * o.y;
-                    up.y += a.beta.x * o.y + a.beta.y * o.x;
-                }
-                Vc[iu] = up;
-            }
-        }
-    }
+        for (int j = 0; j < XS_MT; j++)
+            output(Vc, r0 + mi * XS_MT + i, q0 + mj * XS_MT + j, acc[i][j]);
 }
 
 mdt_status xengine_simt_f32(int ne, long nbatch, int nsp, const float2 *X,
@@ -345,10 +374,10 @@ mdt_status xengine_simt_f32(int ne, long nbatch, int nsp, const float2 *X,
     }
     long blocks = a.dual ? (nbatch + 1) / 2 : nbatch * a.npairs;
     if (blocks > 0x7fffffffL) return invalid("xengine: grid too large");
-    cudaError_t e = cudaFuncSetAttribute(xengine_herm_f32_kernel,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XS_SMEM);
+    auto kern = a.dual && ne <= 28 ? xengine_herm_f32_kernel<true> : xengine_herm_f32_kernel<false>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XS_SMEM);
     if (e != cudaSuccess) return cuda_status(e, "xengine smem attribute");
-    xengine_herm_f32_kernel<<<(unsigned)blocks, XS_THREADS, XS_SMEM, stream>>>(a);
+    kern<<<(unsigned)blocks, XS_THREADS, XS_SMEM, stream>>>(a);
     return launch_status("xengine_herm_f32_kernel");
 }
 
