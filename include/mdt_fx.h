@@ -493,6 +493,12 @@ MDT_API mdt_status mdt_write_binary(const char *path, int nelements, int npols, 
 MDT_API mdt_status mdt_apply_gains(int ne, int nch, int nsp, const void *X, const void *gains,
                                    void *Y, cudaStream_t stream);
 
+/* mdt_fengine_f32 and mdt_apply_gains in one pass, with the same bits: X (null:
+ * not wanted) and Y. */
+MDT_API mdt_status mdt_fengine_gains_f32(int ne, int nch, int ntaps, int nsp, const int8_t *iq,
+                                         const float *window, const void *gains, void *X, void *Y,
+                                         cudaStream_t stream);
+
 /* X-engine adjoint: for V_c = scale * Y_c Y_c^H (mdt_xengine_f32, Y_c =
  * NE x Nsp, stored Y[c][s][e]) and G = grad(V) in the same column-major
  * visibility layout (G[c][q*NE + r] = G_rq),

@@ -6,7 +6,7 @@ Forward (FP32, the plan's arithmetic):
     X = F-engine(iq; taps)      mdt_fengine_f32: PpS_Batch -> FFT -> reorder
                                 (reference MDT_device_functions.cu PpS_Batch,
                                 MDT_OneStation_client.cu:1083-1114)
-    Y = diag(gains) X           mdt_apply_gains, gains [Nch][NE] complex
+    Y = diag(gains) X           mdt_fengine_gains_f32, gains [Nch][NE] complex
     V = Y Y^H / Nsp             mdt_xengine_f32 (replaces cublasCgemmBatched,
                                 MDT_OneStation_client.cu:1128)
 Backward (hand-written adjoints, no PyTorch math on the path):
@@ -28,12 +28,6 @@ def _cplx(n, device):
     return torch.empty(n, dtype=torch.complex64, device=device)
 
 
-def _fengine(iq, taps, ne, nch, ntaps, nsp):
-    X = _cplx(nch * nsp * ne, iq.device)
-    B.fengine_f32(ne, nch, ntaps, nsp, iq, taps, X)
-    return X
-
-
 class FxCorrelate(torch.autograd.Function):
     """V[c, q, r] = (1/Nsp) sum_s Y[c,s,r] conj(Y[c,s,q]),  Y = gains * F(iq; taps).
 
@@ -49,10 +43,8 @@ class FxCorrelate(torch.autograd.Function):
         gains = gains.detach().contiguous().to(torch.complex64)
         if taps.numel() != ntaps * nch or gains.numel() != nch * ne:
             raise B.MdtError("FxCorrelate: taps must hold Ntaps*Nch and gains Nch*NE values")
-        X = _fengine(iq, taps, ne, nch, ntaps, nsp)
-        Y = torch.empty_like(X)
-        B.apply_gains(ne, nch, nsp, X, gains, Y)
-        del X
+        Y = _cplx(nch * nsp * ne, iq.device)
+        B.fengine_gains_f32(ne, nch, ntaps, nsp, iq, taps, gains, Y)
         V = torch.empty(nch, ne, ne, dtype=torch.complex64, device=iq.device)
         B.xengine_f32(ne, nch, nsp, Y, ne, nsp * ne, 1.0 / nsp, V)
         ctx.save_for_backward(iq, taps, gains)
@@ -67,19 +59,20 @@ class FxCorrelate(torch.autograd.Function):
         if not (need_taps or need_gains):
             return (None,) * 7
         G = gV.detach().to(torch.complex64).contiguous()
-        X = _fengine(iq, taps, ne, nch, ntaps, nsp)  # recomputed, not stored
-        Y = torch.empty_like(X)
-        B.apply_gains(ne, nch, nsp, X, gains, Y)
-        dY = torch.empty_like(X)
+        # recomputed, not stored; X is wanted for the gain gradient alone
+        Y = _cplx(nch * nsp * ne, iq.device)
+        X = torch.empty_like(Y) if need_gains else None
+        B.fengine_gains_f32(ne, nch, ntaps, nsp, iq, taps, gains, Y, X=X)
+        dY = torch.empty_like(Y)
         B.xengine_adjoint_f32(ne, nch, nsp, G, Y, dY, 1.0 / nsp)
         dgains = torch.empty(nch, ne, dtype=torch.complex64, device=iq.device) \
             if need_gains else None
         dF = Y if need_taps else None  # Y is dead from here on: reuse it
-        B.gain_adjoint(ne, nch, nsp, dY, X=X if need_gains else None, gains=gains,
+        B.gain_adjoint(ne, nch, nsp, dY, X=X, gains=gains,
                        dgains=dgains, dF=dF)
+        del X
         dtaps = None
         if need_taps:
-            del X
             dP = dY  # dY is consumed: the inverse FFT writes over it
             B.fft_c2c(dF, dP, nsp * ne, nch, B.CUFFT_INVERSE)
             dtaps = torch.empty(ntaps * nch, dtype=torch.float32, device=iq.device)

@@ -110,6 +110,7 @@ def _declare(L):
                                  ctypes.POINTER(ctypes.c_longlong),
                                  ctypes.POINTER(ctypes.c_longlong),
                                  ctypes.POINTER(ctypes.c_size_t)], _I),
+        "mdt_fengine_gains_f32": ([_I, _I, _I, _I, _P, _P, _P, _P, _P, _P], _I),
         "mdt_apply_gains": ([_I, _I, _I, _P, _P, _P, _P], _I),
         "mdt_xengine_adjoint_f32": ([_I, _I, _I, _P, _P, _P, _F, _P], _I),
         "mdt_gain_adjoint": ([_I, _I, _I, _P, _P, _P, _P, _P, _P], _I),
@@ -509,6 +510,12 @@ def write_binary(path, nelements, npols, nch, formatted, append=False):
 def apply_gains(ne, nch, nsp, X, gains, Y, stream=None):
     check(lib().mdt_apply_gains(ne, nch, nsp, ptr(X), ptr(gains), ptr(Y), stream_handle(stream)),
           "apply_gains")
+
+
+def fengine_gains_f32(ne, nch, ntaps, nsp, iq, window, gains, Y, X=None, stream=None):
+    """fengine_f32 and apply_gains in one pass: Y, and X if it is given."""
+    check(lib().mdt_fengine_gains_f32(ne, nch, ntaps, nsp, ptr(iq), ptr(window), ptr(gains), ptr(X),
+                                      ptr(Y), stream_handle(stream)), "fengine_gains_f32")
 
 
 def xengine_adjoint_f32(ne, nch, nsp, G, Y, dY, scale, stream=None):

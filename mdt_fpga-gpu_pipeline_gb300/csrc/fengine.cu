@@ -19,6 +19,7 @@
 #include <cuda_bf16.h>
 #include <algorithm>
 #include <cuda_fp16.h>
+#include <type_traits>
 
 #include "fengine.cuh"
 #include "fft_core.cuh"
@@ -65,6 +66,8 @@ struct FengArgs {
     const float *win;
     const float2 *tw;
     float2 *X;
+    const float2 *gains = nullptr;  // [Nch][NE]: also Y = gains X (then X may be null)
+    float2 *Y = nullptr;
 };
 
 // Two int8 (re, im) samples as packed pairs, without the conversion unit: byte
@@ -138,7 +141,10 @@ __device__ __forceinline__ void pfb_rows_to_smem(const FengArgs &a, long row0, i
     }
 }
 
-template <int N, int R>
+// GAINS: the spectra times the gains as well as, or instead of, the spectra -- a pass over
+// the output less than mdt_apply_gains on it, which is bound by HBM (NE=64, Nch=512,
+// Nsp=2048, 4 taps: Y alone 341 us, X and Y 391; 294 + 158 one after the other).
+template <int N, int R, bool GAINS>
 __global__ void __launch_bounds__(FengCfg<N, R>::THREADS, FengCfg<N, R>::MINB)
     fengine_f32_kernel(FengArgs a)
 {
@@ -158,9 +164,22 @@ __global__ void __launch_bounds__(FengCfg<N, R>::THREADS, FengCfg<N, R>::MINB)
     // corner turn: ROWS contiguous (spectrum, element) rows per channel
     const int nrow = (int)min((long)C::ROWS, rows - row0);
     float2 *dst = a.X + row0;
-    for (int k = threadIdx.x; k < N * C::ROWS; k += C::THREADS) {
-        const int c = k / C::ROWS, r = k - c * C::ROWS;
-        if (r < nrow) dst[(long)c * rows + r] = fsm[(size_t)r * C::RSTRIDE + fft::pad(c)];
+    if constexpr (!GAINS) {
+        for (int k = threadIdx.x; k < N * C::ROWS; k += C::THREADS) {
+            const int c = k / C::ROWS, r = k - c * C::ROWS;
+            if (r < nrow) dst[(long)c * rows + r] = fsm[(size_t)r * C::RSTRIDE + fft::pad(c)];
+        }
+    } else {
+        const int r = threadIdx.x % C::ROWS;  // a thread's rows are all one row
+        if (r >= nrow) return;
+        const float2 *g = a.gains + (row0 + r) % a.ne;
+        float2 *dsty = a.Y + row0;
+#pragma unroll 4
+        for (int c = threadIdx.x / C::ROWS; c < N; c += C::TPR) {
+            const float2 v = fsm[(size_t)r * C::RSTRIDE + fft::pad(c)];
+            if (a.X) dst[(long)c * rows + r] = v;
+            dsty[(long)c * rows + r] = cmul(__ldg(g + (long)c * a.ne), v);
+        }
     }
 }
 
@@ -715,7 +734,9 @@ struct Feng16Run {
         if (!a.tw) return st;
         const long units = (long)a.ne * nkc * 4;
         if (units > 0x7fffffffL) return invalid("fengine_x16: grid too large");
-        auto kern = qscales ? fengine_x16_kernel<N, NT, H, true> : fengine_x16_kernel<N, NT, H, false>;
+        auto kern = fengine_x16_kernel<N, NT, H, false>;
+        if constexpr (std::is_same<H, __half>::value)  // int8 is held in f16
+            if (qscales) kern = fengine_x16_kernel<N, NT, H, true>;
         long grid = 0;
         cudaError_t e = feng_grid<N, NT>(kern, units, &grid);
         if (e != cudaSuccess) return cuda_status(e, "fengine_x16 launch shape");
@@ -881,15 +902,15 @@ static mdt_status launch_feng_rows(FengArgs a, cudaStream_t stream)
     mdt_status st;
     a.tw = fft_twiddles(N, &st);
     if (!a.tw) return st;
+    auto kern = a.gains ? fengine_f32_kernel<N, R, true> : fengine_f32_kernel<N, R, false>;
     if (C::SMEM > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(fengine_f32_kernel<N, R>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)C::SMEM);
         if (e != cudaSuccess) return cuda_status(e, "fengine smem attribute");
     }
     const long blocks = cdiv((long)a.nsp * a.ne, C::ROWS);
     if (blocks > 0x7fffffffL) return invalid("fengine: grid too large");
-    fengine_f32_kernel<N, R><<<(unsigned)blocks, C::THREADS, C::SMEM, stream>>>(a);
+    kern<<<(unsigned)blocks, C::THREADS, C::SMEM, stream>>>(a);
     return launch_status("fengine_f32_kernel");
 }
 
@@ -901,7 +922,8 @@ static mdt_status launch_feng(const FengArgs &a, cudaStream_t stream)
 }
 
 mdt_status fengine_f32(int ne, int nch, int ntaps, int nsp, const int8_t *hist, int nhist,
-                       const int8_t *iq, const float *win, float2 *X, cudaStream_t stream)
+                       const int8_t *iq, const float *win, float2 *X, cudaStream_t stream,
+                       const float2 *gains, float2 *Y)
 {
     // the tap sum reads 16-byte vectors of samples and window coefficients
     if (((uintptr_t)iq | (uintptr_t)hist | (uintptr_t)win) & 15)
@@ -915,6 +937,8 @@ mdt_status fengine_f32(int ne, int nch, int ntaps, int nsp, const int8_t *hist, 
     a.nsp = nsp;
     a.win = win;
     a.X = X;
+    a.gains = gains;
+    a.Y = Y;
     switch (nch) {
         case 32: return launch_feng<32>(a, stream);
         case 64: return launch_feng<64>(a, stream);
@@ -988,5 +1012,18 @@ extern "C" MDT_API mdt_status mdt_fengine_f32(int ne, int nch, int ntaps, int ns
     mdt_status st = mdt::check_dims(ne, nch, ntaps, nsp);
     if (st != MDT_SUCCESS) return st;
     if (!iq || !window || !X) return mdt::invalid("fengine_f32: null pointer");
-    return mdt::fengine_f32(ne, nch, ntaps, nsp, nullptr, 0, iq, window, (float2 *)X, stream);
+    return mdt::fengine_f32(ne, nch, ntaps, nsp, nullptr, 0, iq, window, (float2 *)X, stream, nullptr,
+                            nullptr);
+}
+
+extern "C" MDT_API mdt_status mdt_fengine_gains_f32(int ne, int nch, int ntaps, int nsp,
+                                                    const int8_t *iq, const float *window,
+                                                    const void *gains, void *X, void *Y,
+                                                    cudaStream_t stream)
+{
+    mdt_status st = mdt::check_dims(ne, nch, ntaps, nsp);
+    if (st != MDT_SUCCESS) return st;
+    if (!iq || !window || !gains || !Y) return mdt::invalid("fengine_gains_f32: null pointer");
+    return mdt::fengine_f32(ne, nch, ntaps, nsp, nullptr, 0, iq, window, (float2 *)X, stream,
+                            (const float2 *)gains, (float2 *)Y);
 }

@@ -17,7 +17,8 @@
 namespace mdt {
 mdt_status check_dims(int ne, int nch, int ntaps, int nsp);
 mdt_status fengine_f32(int ne, int nch, int ntaps, int nsp, const int8_t *hist, int nhist,
-                       const int8_t *iq, const float *win, float2 *X, cudaStream_t stream);
+                       const int8_t *iq, const float *win, float2 *X, cudaStream_t stream,
+                       const float2 *gains = nullptr, float2 *Y = nullptr);
 mdt_status fengine_c64b(int ne, int nch, int ntaps, int nsp, const int8_t *hist, int nhist,
                         const int8_t *iq, const float *win, float2 *XB, cudaStream_t stream);
 const float2 *fft_twiddles(int n, mdt_status *st);

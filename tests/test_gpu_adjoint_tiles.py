@@ -62,3 +62,21 @@ def test_tap_grad_runs(mdt, cuda, ntaps, ne, nch, nsp):
                      for i in range(ntaps)])
     got = gW.cpu().numpy()
     assert np.all(np.abs(got - want) <= 2.0 ** -24 * np.abs(want) + 2.0 ** -40 * size)
+
+
+@pytest.mark.parametrize("ne,nch,ntaps,nsp", [(3, 32, 4, 3), (5, 64, 8, 7), (11, 512, 4, 386),
+                                              (16, 2048, 5, 40), (3, 4096, 16, 9)])
+def test_fengine_with_gains(mdt, cuda, ne, nch, ntaps, nsp):
+    """One pass gives the bits of the F-engine and of the gains on its output."""
+    rng = np.random.default_rng(nch + ne)
+    iq = dev(rng.integers(-128, 128, (nsp + ntaps - 1, ne, nch, 2)).astype(np.int8))
+    win = dev(rng.standard_normal(ntaps * nch).astype(np.float32))
+    g = dev(crandn(rng, nch, ne).astype(np.complex64))
+    X, Y, X2, Y2, Y3 = (torch.full((nch, nsp, ne), float("nan"), dtype=torch.complex64,
+                                   device="cuda") for _ in range(5))
+    mdt.fengine_f32(ne, nch, ntaps, nsp, iq, win, X)
+    mdt.apply_gains(ne, nch, nsp, X, g, Y)
+    mdt.fengine_gains_f32(ne, nch, ntaps, nsp, iq, win, g, Y2, X=X2)
+    mdt.fengine_gains_f32(ne, nch, ntaps, nsp, iq, win, g, Y3)
+    for a, b in ((X, X2), (Y, Y2), (Y, Y3)):
+        assert torch.equal(torch.view_as_real(a), torch.view_as_real(b))
