@@ -253,7 +253,10 @@ def kernel_roofline(cfg, precision, f_ms, x_ms, sm_mhz, nsm, fp32_peak=None):
     if precision == "fp32":
         f_bytes = (nsp + ntaps - 1) * sb + nsp * ne * nch * 8 + ntaps * nch * 4
         x_bytes = nsp * ne * nch * 8 + nch * ne * ne * 8
-        fname, xname, xbound = "fengine_c64b", "xengine_herm_f32", "fp32"
+        # from 256 spectra on the X-engine's products run as split f16 pairs on the tensor
+        # cores: the FP32 FMA rate is then a comparison, not its bound
+        split = nsp >= 256
+        fname, xname, xbound = "fengine_c64b", "xengine_f32" if split else "xengine_herm_f32", "fp32"
         xpeak = nsm * 128 * 2 * (sm_mhz or 1900.0) * 1e6 / 1e12
         xpeak_src = ("nominal FP32 FMA rate (%d SMs x 128 lanes x 2) at the sampled SM clock"
                      % nsm)
@@ -261,6 +264,8 @@ def kernel_roofline(cfg, precision, f_ms, x_ms, sm_mhz, nsm, fp32_peak=None):
             xpeak = fp32_peak
             xpeak_src = ("measured FP32 FMA rate (mdt_fp32_peak: one 1024-thread CTA per SM, "
                          "independent FMA chains, the faster of packed f32x2 and scalar)")
+        if split:
+            xpeak_src += "; the kernel computes on the tensor cores, so no bound of it"
         traffic = NCU_TRAFFIC_C2 if cfg.name == "c2_station40" else {}
     else:
         nep, nkc = (ne + 15) // 16 * 16, (nsp + 31) // 32
@@ -746,8 +751,8 @@ def paths_section(mdt, cfg, dev, iq, win, main_ms, main_precision, steps):
     v32 = one.antenna_samples() / (ms32 * 1e-3)
     res["fp32_path"] = {"value": v32, "unit": "antenna-samples/s", "ms_per_integration": ms32,
                         "fengine_ms": f32, "xengine_ms": x32,
-                        "note": "one integration of the same stream (the X-engine is FP32 "
-                                "SIMT; its speed does not depend on the integration)"}
+                        "note": "one integration of the same stream (its speed does "
+                                "not depend on the integration)"}
     main_value = samples / (main_ms * 1e-3)
     res["speedup_vs_fp32_path"] = {main_precision: main_value / v32}
     for k in ("fp16", "bf16", "int8"):

@@ -14,9 +14,10 @@
  *     cublasCreate/cublasSetStream/cublasCgemmBatched subset that the
  *     reference client calls (MDT_OneStation_client.cu:622,630,1105,690,699,
  *     1128), implemented on this library's own kernels.  The mdt_launch_*
- *     functions below launch the drop-in kernels with a caller-chosen grid,
- *     exactly as the reference client's <<<grid, block, 0, stream>>> does,
- *     for callers (ctypes, other languages) that cannot use <<<>>>.
+ *     functions below take a grid as the reference client's
+ *     <<<grid, block, 0, stream>>> does, for callers (ctypes, other languages)
+ *     that cannot use <<<>>>; the grid gives the sizes and is checked as a
+ *     launch would check it, the work itself may run on a grid of its own.
  *
  *  2. Stage entry points (mdt_fft_*, mdt_xengine_*, mdt_fengine_*): one hot
  *     stage each, on caller-allocated device buffers.
@@ -124,7 +125,8 @@ MDT_API mdt_status mdt_window_hamming_sinc(int nchannels, int ntaps, float *wind
 MDT_API mdt_status mdt_fft_c2c(const void *in, void *out, long rows, int n, int direction,
                                cudaStream_t stream);
 
-/* Hermitian X-engine, FP32 SIMT:  for each channel c,
+/* Hermitian X-engine, FP32 (from 256 spectra on as exact products of split
+ * samples on the tensor cores, else SIMT):  for each channel c,
  *   V_c = alpha * X_c X_c^H   (X_c = NE x Nsp column-major with leading
  *   dimension ld >= NE, base X + c*xstride complex values), written full square
  *   column-major with leading dimension NE at V + c*NE*NE.  Only the lower
@@ -242,7 +244,7 @@ MDT_API mdt_status mdt_synth_iq(uint64_t seed, int ne, int nch, long s0, long ns
  * ---------------------------------------------------------------------- */
 
 typedef enum {
-    MDT_PREC_FP32 = 0, /* complex64 F-output, FP32 SIMT X-engine (<=1e-5 vs FP64) */
+    MDT_PREC_FP32 = 0, /* complex64 F-output, FP32 X-engine (<=1e-5 vs FP64) */
     MDT_PREC_FP16 = 1, /* f16 F-output (power-of-two scaled), tcgen05 X-engine, FP32
                           accumulate (<=1e-3 vs FP64); Nch <= 2048 */
     MDT_PREC_BF16 = 2, /* as FP16 with bf16 operands */
@@ -272,7 +274,9 @@ MDT_API mdt_status mdt_fx_set_stream(mdt_fx_plan plan, cudaStream_t stream);
 MDT_API mdt_status mdt_fx_set_window(mdt_fx_plan plan, const float *window);
 /* FP64 cross-integration accumulation: when `acc` (device, complex128
  * [Nch][NE*NE], 16-byte aligned, zeroed by the caller) is set, every
- * integration's visibilities are also added into it; NULL disables. */
+ * integration's visibilities are also added into it; NULL disables.  An FP32
+ * plan then computes them on the SIMT cores whatever its size, so that a sum
+ * kept from before continues with terms rounded the same way. */
 MDT_API mdt_status mdt_fx_set_accumulator(mdt_fx_plan plan, void *acc);
 /* INT8 plans: per-channel requantisation scales (device, Nch floats).  The
  * F-output x of channel c becomes clamp(rint(x * scales[c]), -127, 127);

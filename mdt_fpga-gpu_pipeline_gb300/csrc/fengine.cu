@@ -3,7 +3,7 @@
 // ReorderFOutput as three passes over HBM, MDT_OneStation_client.cu:1083,
 // 1105,1114).
 //
-// A block transforms ROWS rows (spectrum s, elements e0..e0+ROWS-1):
+// A block transforms ROWS consecutive (spectrum, element) rows:
 //  * the tap sum P[c] = sum_i W[i*Nch + c] * iq[s+i][e][c] is formed with
 //    16-byte vector loads into shared memory, accumulated with fmaf from zero
 //    in increasing i, the order of PpS_Batch (MDT_device_functions.cu:143-152),
@@ -11,7 +11,7 @@
 //  * the FFT passes run in shared memory (fft_core.cuh), the last one leaves
 //    the spectrum in natural order in shared memory;
 //  * the block writes X[(c*Nsp + s)*NE + e] (ReorderFOutput's layout,
-//    MDT_device_functions.cu:207): for each channel the ROWS elements are
+//    MDT_device_functions.cu:207): for each channel the ROWS values are
 //    contiguous.
 // Input spectra may come from two buffers: the first `nhist` spectra from
 // `hist` (the PFB history carried between integrations, reference
