@@ -512,7 +512,7 @@ MDT_API mdt_status mdt_xengine_adjoint_f32(int ne, int nch, int nsp, const void 
 
 /* Adjoint of the gains and of the channel-major reorder, given dY:
  *   dgains[c][e] = sum_s dY[c][s][e] conj(X[c][s][e])   (if dgains != NULL;
- *                  double accumulation, fixed order)
+ *                  compensated sums, combined in double in a fixed order)
  *   dF[s][e][c]  = conj(gains[c][e]) dY[c][s][e]         (if dF != NULL;
  *                  gains NULL means unit gains).
  * dF is the gradient of the FFT output rows; mdt_fft_c2c with direction +1
@@ -520,6 +520,11 @@ MDT_API mdt_status mdt_xengine_adjoint_f32(int ne, int nch, int nsp, const void 
 MDT_API mdt_status mdt_gain_adjoint(int ne, int nch, int nsp, const void *dY, const void *X,
                                     const void *gains, void *dgains, void *dF,
                                     cudaStream_t stream);
+
+/* mdt_gain_adjoint's dF and its inverse FFT (mdt_fft_c2c, direction +1) in one
+ * pass, with the same bits: dP[s][e][k], not over dY; Nch <= 2048. */
+MDT_API mdt_status mdt_reorder_adjoint_ifft(int ne, int nch, int nsp, const void *dY,
+                                            const void *gains, void *dP, cudaStream_t stream);
 
 /* PFB tap gradient: with P[s][e][k] = sum_i W[i*Nch + k] in[s+i][e][k]
  * (PpS_Batch, reference MDT_device_functions.cu) and gradP = grad(P)

@@ -12,8 +12,8 @@ Forward (FP32, the plan's arithmetic):
 Backward (hand-written adjoints, no PyTorch math on the path):
     dY     = (G + G^H) Y / Nsp          mdt_xengine_adjoint_f32
     dgains = sum_s dY conj(X)           mdt_gain_adjoint
-    dF     = reorder^T(conj(g) dY)      mdt_gain_adjoint
-    dP     = DFT^H dF                   mdt_fft_c2c(direction=+1)
+    dF     = reorder^T(conj(g) dY)      mdt_reorder_adjoint_ifft (Nch <= 2048),
+    dP     = DFT^H dF                   else mdt_gain_adjoint, mdt_fft_c2c(direction=+1)
     dtaps  = sum Re(dP conj(in))        mdt_pfb_tap_grad
 The F-engine output is recomputed in the backward pass instead of being kept
 from the forward pass (it is Nch*Nsp*NE*8 bytes, the largest tensor here).
@@ -67,14 +67,17 @@ class FxCorrelate(torch.autograd.Function):
         B.xengine_adjoint_f32(ne, nch, nsp, G, Y, dY, 1.0 / nsp)
         dgains = torch.empty(nch, ne, dtype=torch.complex64, device=iq.device) \
             if need_gains else None
-        dF = Y if need_taps else None  # Y is dead from here on: reuse it
-        B.gain_adjoint(ne, nch, nsp, dY, X=X, gains=gains,
-                       dgains=dgains, dF=dF)
+        fused = nch <= 2048  # reorder and FFT in one pass: faster up to there
+        dF = Y if need_taps and not fused else None  # Y is dead from here on: reuse it
+        B.gain_adjoint(ne, nch, nsp, dY, X=X, gains=gains, dgains=dgains, dF=dF)
         del X
         dtaps = None
         if need_taps:
-            dP = dY  # dY is consumed: the inverse FFT writes over it
-            B.fft_c2c(dF, dP, nsp * ne, nch, B.CUFFT_INVERSE)
+            dP = Y if fused else dY
+            if fused:
+                B.reorder_adjoint_ifft(ne, nch, nsp, dY, gains, dP)
+            else:
+                B.fft_c2c(dF, dP, nsp * ne, nch, B.CUFFT_INVERSE)
             dtaps = torch.empty(ntaps * nch, dtype=torch.float32, device=iq.device)
             ws = torch.empty(ntaps * nch * 64, dtype=torch.float64, device=iq.device)
             B.pfb_tap_grad(ne, nch, ntaps, nsp, dP, iq, dtaps, ws)

@@ -110,6 +110,7 @@ def _declare(L):
                                  ctypes.POINTER(ctypes.c_longlong),
                                  ctypes.POINTER(ctypes.c_longlong),
                                  ctypes.POINTER(ctypes.c_size_t)], _I),
+        "mdt_reorder_adjoint_ifft": ([_I, _I, _I, _P, _P, _P, _P], _I),
         "mdt_fengine_gains_f32": ([_I, _I, _I, _I, _P, _P, _P, _P, _P, _P], _I),
         "mdt_apply_gains": ([_I, _I, _I, _P, _P, _P, _P], _I),
         "mdt_xengine_adjoint_f32": ([_I, _I, _I, _P, _P, _P, _F, _P], _I),
@@ -526,6 +527,12 @@ def xengine_adjoint_f32(ne, nch, nsp, G, Y, dY, scale, stream=None):
 def gain_adjoint(ne, nch, nsp, dY, X=None, gains=None, dgains=None, dF=None, stream=None):
     check(lib().mdt_gain_adjoint(ne, nch, nsp, ptr(dY), ptr(X), ptr(gains), ptr(dgains), ptr(dF),
                                  stream_handle(stream)), "gain_adjoint")
+
+
+def reorder_adjoint_ifft(ne, nch, nsp, dY, gains, dP, stream=None):
+    """gain_adjoint's dF and its inverse FFT in one pass; dP is not dY."""
+    check(lib().mdt_reorder_adjoint_ifft(ne, nch, nsp, ptr(dY), ptr(gains), ptr(dP),
+                                         stream_handle(stream)), "reorder_adjoint_ifft")
 
 
 def pfb_tap_grad(ne, nch, ntaps, nsp, gradP, iq, gradW, workspace, stream=None):

@@ -133,6 +133,72 @@ mdt_status fft_c2c(const void *in, void *out, long rows, int n, int direction,
     return MDT_ERR_NOT_SUPPORTED;
 }
 
+// ------------------------------------------------------------ reorder adjoint and inverse
+// dP[row][k] = inverse FFT over c of conj(g[c][row % NE]) dY[c][row], rows = Nsp * NE: the
+// adjoint of gains, corner turn and FFT in one pass.  A block takes up to 8 rows: it reads 64
+// contiguous bytes of each channel into the rows' shared memory and stores the last FFT pass
+// straight to dP.  Bound by HBM (16 bytes a value) and by the latency of its loads: NE=64,
+// Nch=512, Nsp=2048 240 us; mdt_gain_adjoint's dF (212) and then mdt_fft_c2c (169) write and
+// read the values once more.  Nch 2048, Nsp=512 381 us and 408; from 4096 channels on a block
+// has too few rows for whole sectors (467 and 457) and the two calls stay.
+template <int N>
+struct TurnCfg {
+    static constexpr int TPR = N < 256 ? N / 8 : N / 16;
+    static constexpr int ROWS = 1024 / TPR < 8 ? 1024 / TPR : 8;
+    static constexpr int THREADS = ROWS * TPR;
+    static constexpr int RSTRIDE = fft::Shape<N>::PADN + 2;  // rows in different banks
+    static constexpr size_t SMEM = sizeof(float2) * (size_t)RSTRIDE * ROWS;
+};
+
+template <int N>
+__global__ void __launch_bounds__(TurnCfg<N>::THREADS, 1024 / TurnCfg<N>::THREADS)
+    reorder_adjoint_ifft_kernel(int ne, long rows, const float2 *__restrict__ dY,
+                                const float2 *__restrict__ g, float2 *__restrict__ dP,
+                                const float2 *__restrict__ tw)
+{
+    using C = TurnCfg<N>;
+    extern __shared__ float2 smem2[];
+    const long row0 = (long)blockIdx.x * C::ROWS;
+    {
+        const int r = threadIdx.x % C::ROWS;  // a thread's values are all of one row
+        const bool valid = row0 + r < rows;
+        const long row = valid ? row0 + r : 0;
+        const float2 *src = dY + row, *gr = g + row % ne;
+#pragma unroll 8
+        for (int c = threadIdx.x / C::ROWS; c < N; c += C::TPR) {
+            const float2 v = cmul(cconj(__ldg(gr + (long)c * ne)), __ldg(src + (long)c * rows));
+            smem2[r * C::RSTRIDE + fft::pad(c)] = valid ? cconj(v) : make_float2(0.f, 0.f);
+        }
+    }
+    __syncthreads();
+    const int lrow = threadIdx.x / C::TPR, t = threadIdx.x - lrow * C::TPR;
+    const bool valid = row0 + lrow < rows;
+    float2 *dst = dP + (valid ? row0 + lrow : 0) * N;
+    auto none_load = [](int) { return make_float2(0.f, 0.f); };
+    auto store = [&](int i, float2 v) {
+        if (valid) dst[i] = cconj(v);
+    };
+    fft::transform_row<N, C::TPR, false, true>(smem2 + (size_t)lrow * C::RSTRIDE, t, tw, none_load, store);
+}
+
+template <int N>
+static mdt_status launch_turn(int ne, long rows, const float2 *dY, const float2 *g, float2 *dP,
+                              cudaStream_t stream)
+{
+    using C = TurnCfg<N>;
+    mdt_status st;
+    const float2 *tw = fft_twiddles(N, &st);
+    if (!tw) return st;
+    cudaError_t e = cudaFuncSetAttribute(reorder_adjoint_ifft_kernel<N>,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::SMEM);
+    if (e != cudaSuccess) return cuda_status(e, "reorder_adjoint_ifft smem attribute");
+    const long blocks = cdiv(rows, C::ROWS);
+    if (blocks > 0x7fffffffL) return invalid("reorder_adjoint_ifft: too many rows");
+    reorder_adjoint_ifft_kernel<N><<<(unsigned)blocks, C::THREADS, C::SMEM, stream>>>(ne, rows, dY, g,
+                                                                                     dP, tw);
+    return launch_status("reorder_adjoint_ifft_kernel");
+}
+
 // ------------------------------------------------------------ cuFFT subset
 struct ShimPlan {
     int n = 0;
@@ -151,6 +217,27 @@ MDT_API mdt_status mdt_fft_c2c(const void *in, void *out, long rows, int n, int 
                                cudaStream_t stream)
 {
     return mdt::fft_c2c(in, out, rows, n, direction, stream);
+}
+
+MDT_API mdt_status mdt_reorder_adjoint_ifft(int ne, int nch, int nsp, const void *dY,
+                                            const void *gains, void *dP, cudaStream_t stream)
+{
+    if (!dY || !gains || !dP || dY == dP || ne < 1 || nsp < 1)
+        return mdt::invalid("reorder_adjoint_ifft: bad arguments");
+    const long rows = (long)nsp * ne;
+    const float2 *y = (const float2 *)dY, *g = (const float2 *)gains;
+    float2 *p = (float2 *)dP;
+    switch (nch) {
+        case 32: return mdt::launch_turn<32>(ne, rows, y, g, p, stream);
+        case 64: return mdt::launch_turn<64>(ne, rows, y, g, p, stream);
+        case 128: return mdt::launch_turn<128>(ne, rows, y, g, p, stream);
+        case 256: return mdt::launch_turn<256>(ne, rows, y, g, p, stream);
+        case 512: return mdt::launch_turn<512>(ne, rows, y, g, p, stream);
+        case 1024: return mdt::launch_turn<1024>(ne, rows, y, g, p, stream);
+        case 2048: return mdt::launch_turn<2048>(ne, rows, y, g, p, stream);
+        default: break;
+    }
+    return mdt::invalid("reorder_adjoint_ifft: Nch must be a power of two in [32, 2048]");
 }
 
 // cufftPlan1d(&plan, Nch, CUFFT_C2C, Nspectra*Npols*Nelements)

@@ -80,3 +80,18 @@ def test_fengine_with_gains(mdt, cuda, ne, nch, ntaps, nsp):
     mdt.fengine_gains_f32(ne, nch, ntaps, nsp, iq, win, g, Y3)
     for a, b in ((X, X2), (Y, Y2), (Y, Y3)):
         assert torch.equal(torch.view_as_real(a), torch.view_as_real(b))
+
+
+@pytest.mark.parametrize("ne,nch,nsp", [(1, 32, 3), (5, 64, 7), (3, 128, 5), (11, 256, 33),
+                                        (64, 512, 9), (7, 1024, 10), (3, 2048, 11)])
+def test_reorder_adjoint_with_ifft(mdt, cuda, ne, nch, nsp):
+    """One pass gives the bits of the reorder's adjoint and the inverse FFT of it."""
+    rng = np.random.default_rng(nch + ne)
+    dY = dev(crandn(rng, nch, nsp, ne).astype(np.complex64))
+    g = dev(crandn(rng, nch, ne).astype(np.complex64))
+    dF, dP, got = (torch.full((nsp, ne, nch), float("nan"), dtype=torch.complex64, device="cuda")
+                   for _ in range(3))
+    mdt.gain_adjoint(ne, nch, nsp, dY, gains=g, dF=dF)
+    mdt.fft_c2c(dF, dP, nsp * ne, nch, 1)
+    mdt.reorder_adjoint_ifft(ne, nch, nsp, dY, g, got)
+    assert torch.equal(torch.view_as_real(got), torch.view_as_real(dP))
