@@ -160,6 +160,10 @@ __global__ void __launch_bounds__(32 * DP_WARPS)
         const uint32_t *hdr = (const uint32_t *)(pkts + pk * g.pkt_bytes);
         const uint32_t station = __ldg(hdr), snap = __ldg(hdr + 1), counter = __ldg(hdr + 2);
         const long long slot = (long long)counter - g.c0;
+        // this packet's copy has landed, also where the packet is then rejected: the
+        // next iteration issues a copy into the same buffer, and copies of different
+        // groups may land in any order
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
         if (snap >= (uint32_t)g.nsnap || station >= (uint32_t)g.nstation ||
             (long)station * g.ips + g.snap_off[snap] + g.snap_n[snap] > g.ne) {
             if (lane == 0) atomicAdd(&s_cnt[2], 1u);
@@ -186,8 +190,6 @@ __global__ void __launch_bounds__(32 * DP_WARPS)
                 copy_words<WB>(buf, pay + pk * g.pkt_bytes + (long)i0 * nin * per,
                                (ns * nin * per + WB - 1) / WB, lane);
                 asm volatile("cp.async.wait_group 0;" ::: "memory");
-            } else {
-                asm volatile("cp.async.wait_group 1;" ::: "memory");
             }
             __syncwarp();
             const long long s = first + i0 + lane;
