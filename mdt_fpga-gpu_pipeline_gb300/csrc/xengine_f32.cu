@@ -1,5 +1,5 @@
 // xengine_f32.cu -- FP32 Hermitian X-engine on the tensor cores: per channel c
-//   V_c = alpha * X_c X_c^H (+ beta V_c)
+//   V_c = alpha * X_c X_c^H
 // on the lower triangle, mirrored; the reference's cublasCgemmBatched call
 // (OP_N, OP_C, A == B, alpha = 1/Nspectra, beta = 0;
 // MDT_OneStation_client.cu:1128, :656-660, :683-686).
@@ -22,11 +22,22 @@
 //   NE=10, Nsp=1000: 5.8e-8, 9.2e-8;   NE=40, Nsp=512: 7.1e-8, 2.4e-7;
 //   NE=40, Nsp=4096: 6.0e-8, 6.2e-7;   NE=256, Nsp=2048: 7.9e-8, 8.8e-7.
 //
-// Samples or products that are not finite make the affected sums NaN; every
-// visibility that comes out non-finite is formed again by FP32 multiply-adds
-// over its two elements, so infinities and NaN appear as that sum gives
-// them.  A block whose waits gave up (each is bounded) forms its whole tile
-// that way.
+// Where it does not hold.  The rest is rounded on the grid of the largest component, so
+// samples far below it lose bits that FP32 would keep; if the other element is zero where
+// the large ones are (a burst in one element, spectra lost in the other), nothing makes up
+// for it: a spectrum of 64 that is 2^10 above the others cost 5e-6 of such a visibility,
+// 2^16 2e-5.  So on the diagonal tiles the kernel counts for each element and stage the
+// spectra with a component within 2^-4 (at most 2^-5) of the largest; where a quarter or
+// more are below, or the largest is outside [2^-48, 2^48], it leaves a mark
+// for the element (xf_mark), and xengine_simt_redo forms all its visibilities by FP32
+// multiply-adds.  Two elements that pass share half the spectra of every stage well above
+// the grid.  (Normal noise fails less than once in 10^9 stages; an element that is zero
+// throughout a stage passes, its products are exact.)
+//
+// Samples that are not finite make the affected sums NaN; every visibility that comes out
+// non-finite is formed again by FP32 multiply-adds over its two elements, so infinities
+// and NaN appear as that sum gives them.  A block whose waits gave up (each is bounded)
+// forms its whole tile that way.
 //
 // Layout of the products: re and im of an element are separate rows of one real
 // operand Z (2 nb rows, nb = elements rounded up to 8), and D = Z Z^T holds
@@ -42,15 +53,15 @@
 // the K-major 128-byte-swizzled operand, and adds the sums of an earlier stage from
 // tensor memory to its registers.  Two operand stages and two accumulator sets
 // alternate: while the tensor core works on stage k + 1, the warps drain stage k
-// and write stage k + 2 over its operands.
+// and write stage k + 2 over its operands.  Five warpgroups share the registers: 104 for
+// a converting thread instead of 96, without which the count spills.
 //
 // What bounds it: an M = 128, K = 16 MMA takes 63 cycles for any N up to 128, so the
-// sixteen of a stage take 1000 of the 2200 to 3000 cycles that a stage takes; the
-// rest is the warps' chain of tensor-memory reads (about 300 cycles a batch under
-// MMAs), conversion and sample loads, one after the other.  Times, against the
-// SIMT kernel's: NE=256, Nch=1024, Nsp=2048 4.98 ms, 12.53; NE=64, Nch=512, Nsp=2048
-// 0.33, 0.70; NE=38, Nch=Nsp=1024 0.20, 0.28; NE=40, Nch=2048, Nsp=4096 1.35, 1.47;
-// NE=10, Nch=1024, Nsp=1000 0.058, 0.083.
+// sixteen of a stage take 1000 of the 3100 cycles that a stage takes at 40 inputs and of
+// the 4500 at 256; the rest is the warps' chain of tensor-memory reads, conversion and
+// sample loads, one after the other.
+#include <cuda_fp16.h>
+
 #include <algorithm>
 
 #include "tc_ptx.cuh"
@@ -58,8 +69,13 @@
 
 namespace mdt {
 
-constexpr int XF_WARPS = 16;                      // converting warps
-constexpr int XF_THREADS = 32 * (XF_WARPS + 1);   // and the issuing warp
+constexpr int XF_WARPS = 16;  // converting warps; then the issuing one and three without work
+// (registers are split by warpgroups).  The kernel is launched with XF_REGS registers a
+// thread; the converting warps take XF_REGS_CONV and the others keep XF_REGS_REST, the
+// same 61,440 in all.
+constexpr int XF_THREADS = 32 * (XF_WARPS + 4);
+constexpr int XF_REGS = 96, XF_REGS_CONV = 104, XF_REGS_REST = 64;
+static_assert(XF_REGS_CONV * 32 * XF_WARPS + XF_REGS_REST * 32 * 4 <= XF_REGS * XF_THREADS, "register split");
 constexpr int XF_K = 64;                          // spectra per stage
 constexpr int XF_PLANE = 128 * 128;               // 128 rows of 64 f16
 constexpr int XF_OPERAND = 2 * XF_PLANE;          // h, l
@@ -69,6 +85,11 @@ constexpr int XF_FLUSH = 8;                       // stages per first-level sum
 // FP32 multiply-adds (NE=10: 6.7e-8 at 64 spectra, 8.6e-8 at 250), there the split
 // is no closer to the 64-bit sums, and there is little time to gain.
 constexpr int XF_MIN_SPECTRA = 256;
+// A stage of an element is uneven if, of its spectra, a quarter or more have no component
+// of XF_SIG or above in the scale that brings the largest one to [1024, 2048), or if that
+// one is outside [2^-XF_EXP, 2^XF_EXP] (whose products are far from FP32's limits).
+constexpr float XF_SIG = 64.0f;
+constexpr int XF_EXP = 48;
 constexpr int XF_DS = 129;                        // floats per row of the exchanged sums
 constexpr size_t XF_D_BYTES = (size_t)128 * XF_DS * sizeof(float);
 constexpr size_t xf_smem(bool off)
@@ -85,8 +106,7 @@ struct XfArgs {
     float2 *V;
     float2 *const *Vptrs;
     long ldv, vstride;
-    float2 alpha, beta;
-    int beta_zero;
+    float2 alpha;
     long nbatch;
 };
 
@@ -114,6 +134,24 @@ __device__ __noinline__ float2 direct_product(const float2 *Xc, long ld, int nsp
     return v;
 }
 
+// Counts the spectra that have a component of XF_SIG or above, two at a time (re, im:
+// their integers as f16 pairs), from 1024 in the low half and 0 in the high one.
+__device__ __forceinline__ void count_significant(__half2 &n, uint32_t re, uint32_t im)
+{
+    const __half2 a = __habs2(*reinterpret_cast<const __half2 *>(&re));
+    const __half2 b = __habs2(*reinterpret_cast<const __half2 *>(&im));
+    n = __hadd2(n, __hge2(__hmax2(a, b), __float2half2_rn(XF_SIG)));
+}
+
+// Of the eight lanes that hold an element, from their counts (all lanes of the warp).
+__device__ __forceinline__ int total_significant(__half2 n)
+{
+    // 1024 + the lane's count, as f16: the low digits of its bits; a byte for each element
+    const uint32_t mine = __half_as_ushort(__hadd(__low2half(n), __high2half(n))) & 15;
+    const int at = threadIdx.x & 24;
+    return __reduce_add_sync(0xffffffffu, mine << at) >> at & 255;
+}
+
 // OFF: the grid holds tiles below the diagonal (NE > 64), with an operand of
 // their own for the columns.  SLOT: rows of M per channel (128, 64 or 32).
 // BLOCKED: operand X[(k/8)*ld + e*8 + k%8] (blocks of 8 spectra, the last one
@@ -126,6 +164,7 @@ __global__ void __launch_bounds__(XF_THREADS, 1) xengine_f32_kernel(const XfArgs
     __shared__ uint64_t bars[4];  // full[2] (operands written), done[2] (products complete)
     __shared__ uint32_t tmem_slot;
     __shared__ int s_fail;
+    __shared__ bool s_uneven[64];  // elements of a diagonal tile: in one of their stages
     __shared__ __align__(16) float s_inv[4][2][64];  // [stage % 4][operand][element]: 1 / scale
     constexpr int NSLOT = 128 / SLOT, EB = SLOT / 2;  // channels, and elements per channel
     constexpr int STAGE = (OFF ? 2 : 1) * XF_OPERAND;
@@ -163,8 +202,9 @@ __global__ void __launch_bounds__(XF_THREADS, 1) xengine_f32_kernel(const XfArgs
     tc::fence_after_sync();
     const uint32_t tmem = tmem_slot;
 
-    if (warp == XF_WARPS) {
-        if (lane == 0) {
+    if (warp >= XF_WARPS) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(XF_REGS_REST));
+        if (warp == XF_WARPS && lane == 0) {
             // ---------------- MMA issuer: h h' to columns 0..127 of the stage's set,
             // the products with l to columns 128..255
             const int N = (NSLOT - 1) * SLOT + 2 * nb;
@@ -193,6 +233,7 @@ __global__ void __launch_bounds__(XF_THREADS, 1) xengine_f32_kernel(const XfArgs
         }
         __syncwarp();
     } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(XF_REGS_CONV));
         // ---------------- converting warps.  A thread takes element e of channel
         // slot g and the spectra 8 (4 sg + i) + 2 p + {0, 1}, i < 4, of a stage: in
         // the blocked layout four lanes (p) read 64 contiguous bytes, and a warp's
@@ -238,6 +279,7 @@ __global__ void __launch_bounds__(XF_THREADS, 1) xengine_f32_kernel(const XfArgs
                 }
             }
         };
+        // writes the operand rows; on a diagonal tile the lane's count of significant spectra
         auto convert = [&](int k, int op, bool live) {
             // the eight lanes of an element agree on the scale
             float m = 0.0f;
@@ -252,11 +294,14 @@ __global__ void __launch_bounds__(XF_THREADS, 1) xengine_f32_kernel(const XfArgs
             const int bs = min(127 + 10 + 127 - (int)(__float_as_uint(m) >> 23), 253);
             const float sc = __uint_as_float((uint32_t)bs << 23);
             if ((lane & 7) == 0) s_inv[k & 3][op][el] = __uint_as_float((uint32_t)(254 - bs) << 23);
-            if (!live) return;  // rows without an element feed sums that are never read
+            const __half2 none = __floats2half2_rn(1024.f, 0.f), all = __floats2half2_rn(1024.f + 8.f, 0.f);
+            if (!live) return all;  // rows without an element feed sums that are never read
             const float2 sc2 = make_float2(sc, sc);
             const float2 big = make_float2(12582912.0f, 12582912.0f);  // 1.5 * 2^23: rounds to integers
             const float2 nbig = make_float2(-12582912.0f, -12582912.0f);
             uint8_t *st = smem + (size_t)(k & 1) * STAGE + (size_t)op * XF_OPERAND;
+            __half2 nsig = none;
+            uint32_t hre[4];
 #pragma unroll
             for (int c = 0; c < 2; c++) {
                 const int row = g * SLOT + c * nb + e;
@@ -267,9 +312,24 @@ __global__ void __launch_bounds__(XF_THREADS, 1) xengine_f32_kernel(const XfArgs
                     const float2 h = __fadd2_rn(__ffma2_rn(x, sc2, big), nbig);
                     const float2 l = __ffma2_rn(x, sc2, make_float2(-h.x, -h.y));
                     const int at = ((4 * sg + i) ^ (row & 7)) << 4;
-                    *reinterpret_cast<uint32_t *>(w + at) = f16x2(h);
+                    const uint32_t h16 = f16x2(h);
+                    *reinterpret_cast<uint32_t *>(w + at) = h16;
                     *reinterpret_cast<uint32_t *>(w + at + XF_PLANE) = f16x2(l);
+                    if (c == 0)
+                        hre[i] = h16;
+                    else if (!sep)
+                        count_significant(nsig, hre[i], h16);
                 }
+            }
+            if (m == 0.0f) return all;
+            return m >= 1.0f / (1ll << XF_EXP) && m <= (float)(1ll << XF_EXP) ? nsig : none;
+        };
+        bool uneven = false;
+        auto check = [&](int k, __half2 nsig) {
+            const int n = min(XF_K, a.nsp - k * XF_K);
+            if (!sep) {
+                const int sig = total_significant(nsig);  // by all lanes
+                uneven |= sig < n - (n - 1) / 4;
             }
         };
         auto arrive = [&](int k) {  // operands of stage k written, sums of stage k - 2 read
@@ -328,12 +388,13 @@ __global__ void __launch_bounds__(XF_THREADS, 1) xengine_f32_kernel(const XfArgs
         bool ok = true;
         for (int k = 0; k < min(2, nstage); k++) {
             load(xa, liveA, k);
-            convert(k, 0, liveA);
+            const __half2 nsig = convert(k, 0, liveA);
             if (sep) {
                 load(xb, liveB, k);
                 convert(k, 1, liveB);
             }
             arrive(k);
+            check(k, nsig);
         }
         if (nstage > 2) load(xa, liveA, 2);
         for (int k = 0; k < nstage; k++) {
@@ -346,8 +407,9 @@ __global__ void __launch_bounds__(XF_THREADS, 1) xengine_f32_kernel(const XfArgs
             tc::fence_after_sync();
             const bool more = k + 2 < nstage;
             drain(k);
+            __half2 nsig;
             if (more) {
-                convert(k + 2, 0, liveA);
+                nsig = convert(k + 2, 0, liveA);
                 if (sep) load(xb, liveB, k + 2);
             }
             if (k % XF_FLUSH == XF_FLUSH - 1) flush(k < XF_FLUSH);
@@ -355,22 +417,17 @@ __global__ void __launch_bounds__(XF_THREADS, 1) xengine_f32_kernel(const XfArgs
                 if (sep) convert(k + 2, 1, liveB);
                 arrive(k + 2);
                 if (k + 3 < nstage) load(xa, liveA, k + 3);
+                check(k + 2, nsig);
             }
         }
         if (!ok && lane == 0) atomicExch(&s_fail, 1);
         tc::fence_before_sync();
         flush(nstage < XF_FLUSH);
+        if ((lane & 7) == 0) s_uneven[el] = uneven;
         tc::named_barrier(1, 32 * XF_WARPS);
         const bool fail = s_fail != 0;
-        // alpha v + beta V
         auto put = [&](float2 *Vc, long at, float2 v) {
-            float2 o = make_float2(a.alpha.x * v.x - a.alpha.y * v.y, a.alpha.x * v.y + a.alpha.y * v.x);
-            if (!a.beta_zero) {
-                const float2 w = Vc[at];
-                o.x += a.beta.x * w.x - a.beta.y * w.y;
-                o.y += a.beta.x * w.y + a.beta.y * w.x;
-            }
-            Vc[at] = o;
+            Vc[at] = make_float2(a.alpha.x * v.x - a.alpha.y * v.y, a.alpha.x * v.y + a.alpha.y * v.x);
         };
         for (int sl = 0; sl < NSLOT; sl++) {
             const long c = ch0 + sl;
@@ -393,6 +450,7 @@ __global__ void __launch_bounds__(XF_THREADS, 1) xengine_f32_kernel(const XfArgs
                     if (r == q) v.y = 0.f;  // autocorrelations are real
                     if (r < q) v.y = -v.y;
                     put(Vc, (long)(q0 + q) * a.ldv + r0 + r, v);
+                    if (r == q && s_uneven[sl * EB + r]) Vc[(long)(q0 + q) * a.ldv + r0 + r] = xf_mark();
                 }
             } else {
                 for (int i = tid; i < nr * 64; i += 32 * XF_WARPS) {
@@ -414,6 +472,14 @@ __global__ void __launch_bounds__(XF_THREADS, 1) xengine_f32_kernel(const XfArgs
     }
 }
 
+// Whether a launch has the registers that the converting warps take: setmaxnreg waits
+// for ever where it has not.
+static bool split_fits(void (*kern)(const XfArgs))
+{
+    cudaFuncAttributes fa;
+    return cudaFuncGetAttributes(&fa, kern) == cudaSuccess && (fa.numRegs + 7) / 8 * 8 >= XF_REGS;
+}
+
 mdt_status xengine_herm_f32(int ne, long nbatch, int nsp, const float2 *X,
                             const float2 *const *Xptrs, long ld, long xstride, float2 *V,
                             float2 *const *Vptrs, long ldv, long vstride, float2 alpha,
@@ -426,6 +492,10 @@ mdt_status xengine_herm_f32(int ne, long nbatch, int nsp, const float2 *X,
     if (nsp < XF_MIN_SPECTRA || !vectors || ne > (1 << 20))
         return xengine_simt_f32(ne, nbatch, nsp, X, Xptrs, ld, xstride, V, Vptrs, ldv, vstride, alpha,
                                 beta, beta_zero, stream, blocked);
+    // what a visibility was before cannot be added again to one that is formed twice
+    if (!beta_zero)
+        return xengine_simt_redo(ne, nbatch, nsp, X, Xptrs, ld, xstride, V, Vptrs, ldv, vstride, alpha,
+                                 beta, false, true, stream, blocked);
     XfArgs a;
     a.ne = ne;
     a.nsp = nsp;
@@ -440,16 +510,18 @@ mdt_status xengine_herm_f32(int ne, long nbatch, int nsp, const float2 *X,
     a.ldv = ldv;
     a.vstride = vstride;
     a.alpha = alpha;
-    a.beta = beta;
-    a.beta_zero = beta_zero ? 1 : 0;
     a.nbatch = nbatch;
     auto launch = [&](auto kern, bool off, long blocks) -> mdt_status {
         if (blocks > 0x7fffffffL) return invalid("xengine: grid too large");
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)xf_smem(off));
         if (e != cudaSuccess) return cuda_status(e, "xengine smem attribute");
+        if (!split_fits(kern)) return invalid("xengine: compiled with too few registers to split");
         kern<<<(unsigned)blocks, XF_THREADS, xf_smem(off), stream>>>(a);
-        return launch_status("xengine_f32_kernel");
+        const mdt_status st = launch_status("xengine_f32_kernel");
+        if (st != MDT_SUCCESS) return st;
+        return xengine_simt_redo(ne, nbatch, nsp, X, Xptrs, ld, xstride, V, Vptrs, ldv, vstride, alpha,
+                                 make_float2(0.f, 0.f), true, false, stream, blocked);
     };
     if (ne > 64)
         return blocked ? launch(xengine_f32_kernel<true, 128, true>, true, nbatch * a.npairs)

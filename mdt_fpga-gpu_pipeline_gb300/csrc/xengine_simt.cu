@@ -51,6 +51,8 @@ struct XengArgs {
     int beta_zero;
     int blocked;  // operand layout: 0 = X[k*ld + e]; 1 = blocks of 8 samples, X[(k/8)*ld + e*8 + k%8]
     int dual;     // NE <= 64: a block takes two channels (A and B buffers hold one each)
+    int diagonal; // REDO: tiles on the diagonal (1), below it (0)
+    int all;      // REDO: whatever the marks
     long nbatch;
 };
 
@@ -96,8 +98,12 @@ __device__ __forceinline__ int xs_off(int e, int kk)
 // slices each.  Their sums are added by one thread per value instead of one per
 // micro-tile, and fewer rows are staged: NE=10, Nch=1024, Nsp=64 8.3 us, 15.5 without;
 // NE=28, Nsp=16 13.4 and 14.8.  With fewer slices it costs (NE=38, Nsp=64: 31 us, 26).
-template <bool SMALL>
-__global__ void __launch_bounds__(XS_THREADS, 3) xengine_herm_f32_kernel(XengArgs a)
+// REDO: the visibilities of marked elements and tiles (see xf_mark), for the tiles below
+// the diagonal and then for those on it, which hold the marks; most blocks find none and
+// end.  That takes 2 us where there are 512 blocks (4 without the programmatic launch)
+// and 18 us for the 10,240 tiles of NE=256, Nch=1024.
+template <bool SMALL, bool REDO>
+__global__ void __launch_bounds__(XS_THREADS, REDO ? 2 : 3) xengine_herm_f32_kernel(XengArgs a)
 {
     // [stage][operand][k][element]; the K-slice reduction reuses the space
     extern __shared__ float4 xs_smem4[];
@@ -111,10 +117,31 @@ __global__ void __launch_bounds__(XS_THREADS, 3) xengine_herm_f32_kernel(XengArg
     const int pr = a.dual ? 0 : (int)blockIdx.x - ch * a.npairs;
     const bool has2 = a.dual && ch + 1 < a.nbatch;
     int I, J;
-    pair_index(pr, I, J);
+    if (REDO && a.diagonal) {
+        I = J = pr;
+    } else {
+        pair_index(pr, I, J);
+        if (REDO) I++;
+    }
     const bool diag = (I == J);
     const int r0 = I * XS_ST, q0 = J * XS_ST;
     const int nr = min(XS_ST, a.ne - r0), nq = min(XS_ST, a.ne - q0);
+    auto channel = [&](int c) { return a.Vptrs ? a.Vptrs[c] : a.V + (long)c * a.vstride; };
+    __shared__ bool s_redo[2][XS_ST];  // rows and columns, or the rows of two channels
+    if constexpr (REDO) {
+        cudaGridDependencySynchronize();  // the marks are there
+        bool mark = false;
+        if (threadIdx.x < 2 * XS_ST) {
+            const int op = threadIdx.x / XS_ST, e = threadIdx.x % XS_ST;
+            const float2 *Vc = channel(a.dual && has2 ? ch + op : ch);
+            const long at = (a.dual || !op ? r0 : q0) + e;
+            if (e < (a.dual || !op ? nr : nq)) mark = xf_is_mark(Vc[at * (a.ldv + 1)]);
+            if (!diag && !mark) mark = xf_is_mark(Vc[q0 * a.ldv + r0]);
+            mark |= a.all;
+            s_redo[op][e] = mark;
+        }
+        if (!__syncthreads_or(mark)) return;
+    }
     const int nmr = (nr + XS_MT - 1) / XS_MT, nmq = (nq + XS_MT - 1) / XS_MT;
     const int nmt = diag ? nmr * (nmr + 1) / 2 : nmr * nmq;
     const int nmt2 = a.dual ? 2 * nmt : nmt;  // micro-tiles of the block
@@ -188,6 +215,24 @@ __global__ void __launch_bounds__(XS_THREADS, 3) xengine_herm_f32_kernel(XengArg
 #pragma unroll
         for (int j = 0; j < XS_MT; j++) acc[i][j] = make_float2(0.f, 0.f);
 
+    // REDO: sums of 16 spectra, and their sum: one chain of Nsp multiply-adds rounds the
+    // more the longer it is (NE=96, 1024 spectra: 1.5e-6 of a visibility, so 1.0e-7)
+    float2 tot[XS_MT][XS_MT];
+    auto second_level = [&]() {
+#pragma unroll
+        for (int i = 0; i < XS_MT; i++)
+#pragma unroll
+            for (int j = 0; j < XS_MT; j++) {
+                tot[i][j] = __fadd2_rn(tot[i][j], acc[i][j]);
+                acc[i][j] = make_float2(0.f, 0.f);
+            }
+    };
+    if constexpr (REDO) {
+#pragma unroll
+        for (int i = 0; i < XS_MT; i++)
+#pragma unroll
+            for (int j = 0; j < XS_MT; j++) tot[i][j] = make_float2(0.f, 0.f);
+    }
     const int nchunk = (a.nsp + XS_KC - 1) / XS_KC;
     stage(0, 0);
     for (int c = 0; c < nchunk; c++) {
@@ -254,15 +299,24 @@ __global__ void __launch_bounds__(XS_THREADS, 3) xengine_herm_f32_kernel(XengArg
                         acc[i][j].y = fmaf(-av[i].z, bv[j].w, acc[i][j].y);
                     }
 #endif
+                if (REDO && (kp + ksl) / 8 != kp / 8) second_level();
             }
         }
         __syncthreads();  // buffer st is overwritten by the next stage() call
     }
+    if constexpr (REDO) {
+#pragma unroll
+        for (int i = 0; i < XS_MT; i++)
+#pragma unroll
+            for (int j = 0; j < XS_MT; j++) acc[i][j] = tot[i][j];
+    }
 
-    auto channel = [&](int c) { return a.Vptrs ? a.Vptrs[c] : a.V + (long)c * a.vstride; };
     // V[r, q] and its mirror from the sum v over the samples (r >= q)
-    auto output = [&](float2 *Vc, int r, int q, float2 v) {
+    auto output = [&](int c2, int r, int q, float2 v) {
         if (r >= a.ne || q >= a.ne || r < q) return;
+        if (REDO && !(diag ? s_redo[c2][r - r0] || s_redo[c2][q - q0] : s_redo[0][r - r0] || s_redo[1][q - q0]))
+            return;
+        float2 *Vc = channel(ch + c2);
         if (r == q) v.y = 0.f;  // autocorrelations are real
         // lower:  V[r,q] = alpha v + beta V[r,q]
         float2 lo = make_float2(a.alpha.x * v.x - a.alpha.y * v.y,
@@ -309,7 +363,7 @@ __global__ void __launch_bounds__(XS_THREADS, 3) xengine_herm_f32_kernel(XengArg
                 v.x += u.x;
                 v.y += u.y;
             }
-            output(channel(ch + c2), r0 + oi * XS_MT + (ij >> 2), q0 + oj * XS_MT + (ij & 3), v);
+            output(c2, r0 + oi * XS_MT + (ij >> 2), q0 + oj * XS_MT + (ij & 3), v);
         }
         return;
     }
@@ -335,21 +389,18 @@ __global__ void __launch_bounds__(XS_THREADS, 3) xengine_herm_f32_kernel(XengArg
         }
     }
     if (!active || ks != 0) return;
-    float2 *Vc = channel(ch + cs);
 #pragma unroll
     for (int i = 0; i < XS_MT; i++)
 #pragma unroll
         for (int j = 0; j < XS_MT; j++)
-            output(Vc, r0 + mi * XS_MT + i, q0 + mj * XS_MT + j, acc[i][j]);
+            output(cs, r0 + mi * XS_MT + i, q0 + mj * XS_MT + j, acc[i][j]);
 }
 
-mdt_status xengine_simt_f32(int ne, long nbatch, int nsp, const float2 *X,
-                            const float2 *const *Xptrs, long ld, long xstride, float2 *V,
-                            float2 *const *Vptrs, long ldv, long vstride, float2 alpha,
-                            float2 beta, bool beta_zero, cudaStream_t stream, int blocked)
+static XengArgs simt_args(int ne, long nbatch, int nsp, const float2 *X, const float2 *const *Xptrs,
+                          long ld, long xstride, float2 *V, float2 *const *Vptrs, long ldv,
+                          long vstride, float2 alpha, float2 beta, bool beta_zero, int blocked)
 {
-    if (ne <= 0 || nbatch <= 0) return MDT_SUCCESS;
-    XengArgs a;
+    XengArgs a{};
     a.ne = ne;
     a.nsp = nsp;
     a.nsuper = (int)cdiv(ne, XS_ST);
@@ -372,13 +423,60 @@ mdt_status xengine_simt_f32(int ne, long nbatch, int nsp, const float2 *X,
         const int nmr = (int)cdiv(ne, XS_MT);
         a.dual = (a.nsuper == 1 && nmr * (nmr + 1) <= XS_THREADS) ? 1 : 0;
     }
-    long blocks = a.dual ? (nbatch + 1) / 2 : nbatch * a.npairs;
+    return a;
+}
+
+template <bool REDO>
+static mdt_status simt_launch(const XengArgs &a, cudaStream_t stream)
+{
+    const long blocks = a.dual ? (a.nbatch + 1) / 2 : a.nbatch * a.npairs;
     if (blocks > 0x7fffffffL) return invalid("xengine: grid too large");
-    auto kern = a.dual && ne <= 28 ? xengine_herm_f32_kernel<true> : xengine_herm_f32_kernel<false>;
+    auto kern = a.dual && a.ne <= 28 ? xengine_herm_f32_kernel<true, REDO> : xengine_herm_f32_kernel<false, REDO>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)XS_SMEM);
     if (e != cudaSuccess) return cuda_status(e, "xengine smem attribute");
-    kern<<<(unsigned)blocks, XS_THREADS, XS_SMEM, stream>>>(a);
+    // REDO: set up while the kernel before it ends
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3(XS_THREADS);
+    cfg.dynamicSmemBytes = XS_SMEM;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = REDO ? 1 : 0;
+    e = cudaLaunchKernelEx(&cfg, kern, a);
+    if (e != cudaSuccess) return cuda_status(e, "xengine_herm_f32_kernel");
     return launch_status("xengine_herm_f32_kernel");
+}
+
+mdt_status xengine_simt_f32(int ne, long nbatch, int nsp, const float2 *X,
+                            const float2 *const *Xptrs, long ld, long xstride, float2 *V,
+                            float2 *const *Vptrs, long ldv, long vstride, float2 alpha,
+                            float2 beta, bool beta_zero, cudaStream_t stream, int blocked)
+{
+    if (ne <= 0 || nbatch <= 0) return MDT_SUCCESS;
+    return simt_launch<false>(simt_args(ne, nbatch, nsp, X, Xptrs, ld, xstride, V, Vptrs, ldv, vstride, alpha,
+                                        beta, beta_zero, blocked),
+                              stream);
+}
+
+mdt_status xengine_simt_redo(int ne, long nbatch, int nsp, const float2 *X, const float2 *const *Xptrs,
+                             long ld, long xstride, float2 *V, float2 *const *Vptrs, long ldv,
+                             long vstride, float2 alpha, float2 beta, bool beta_zero, bool all,
+                             cudaStream_t stream, int blocked)
+{
+    XengArgs a = simt_args(ne, nbatch, nsp, X, Xptrs, ld, xstride, V, Vptrs, ldv, vstride, alpha, beta,
+                           beta_zero, blocked);
+    a.all = all;
+    if (a.nsuper > 1) {  // the marks stand on the diagonal until these are done
+        a.npairs = a.nsuper * (a.nsuper - 1) / 2;
+        const mdt_status st = simt_launch<true>(a, stream);
+        if (st != MDT_SUCCESS) return st;
+    }
+    a.diagonal = 1;
+    a.npairs = a.nsuper;
+    return simt_launch<true>(a, stream);
 }
 
 // ---------------------------------------------------- general batched CGEMM
