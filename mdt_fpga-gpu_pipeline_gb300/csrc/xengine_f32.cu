@@ -28,16 +28,13 @@
 // for it: a spectrum of 64 that is 2^10 above the others cost 5e-6 of such a visibility,
 // 2^16 2e-5.  So on the diagonal tiles the kernel counts for each element and stage the
 // spectra with a component within 2^-4 (at most 2^-5) of the largest; where a quarter or
-// more are below, or the largest is outside [2^-48, 2^48], it leaves a mark
+// more are below, or the largest is outside [2^-48, 2^48] or not finite, it leaves a mark
 // for the element (xf_mark), and xengine_simt_redo forms all its visibilities by FP32
 // multiply-adds.  Two elements that pass share half the spectra of every stage well above
 // the grid.  (Normal noise fails less than once in 10^9 stages; an element that is zero
-// throughout a stage passes, its products are exact.)
-//
-// Samples that are not finite make the affected sums NaN; every visibility that comes out
-// non-finite is formed again by FP32 multiply-adds over its two elements, so infinities
-// and NaN appear as that sum gives them.  A block whose waits gave up (each is bounded)
-// forms its whole tile that way.
+// throughout a stage passes, its products are exact.)  Infinities and NaN appear as those
+// multiply-adds give them.  A block whose waits gave up (each is bounded) leaves its whole
+// tile to them.
 //
 // Layout of the products: re and im of an element are separate rows of one real
 // operand Z (2 nb rows, nb = elements rounded up to 8), and D = Z Z^T holds
@@ -118,20 +115,12 @@ __device__ __forceinline__ uint32_t f16x2(float2 v)
     return r;
 }
 
-// V_rq by multiply-adds in spectrum order (results that are not finite).
-template <bool BLOCKED>
-__device__ __noinline__ float2 direct_product(const float2 *Xc, long ld, int nsp, int r, int q)
+// The larger of two values; NaN if one of them is.
+__device__ __forceinline__ float max_nan(float a, float b)
 {
-    float2 v = make_float2(0.f, 0.f);
-    for (int k = 0; k < nsp; k++) {
-        const float2 a = BLOCKED ? Xc[(long)(k >> 3) * ld + (long)r * 8 + (k & 7)] : Xc[(long)k * ld + r];
-        const float2 b = BLOCKED ? Xc[(long)(k >> 3) * ld + (long)q * 8 + (k & 7)] : Xc[(long)k * ld + q];
-        v.x = fmaf(a.x, b.x, v.x);
-        v.x = fmaf(a.y, b.y, v.x);
-        v.y = fmaf(a.y, b.x, v.y);
-        v.y = fmaf(-a.x, b.y, v.y);
-    }
-    return v;
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
 }
 
 // Counts the spectra that have a component of XF_SIG or above, two at a time (re, im:
@@ -285,11 +274,11 @@ __global__ void __launch_bounds__(XF_THREADS, 1) xengine_f32_kernel(const XfArgs
             float m = 0.0f;
 #pragma unroll
             for (int i = 0; i < 4; i++) {
-                m = fmaxf(m, fmaxf(fabsf(re[i].x), fabsf(re[i].y)));
-                m = fmaxf(m, fmaxf(fabsf(im[i].x), fabsf(im[i].y)));
+                m = max_nan(m, max_nan(fabsf(re[i].x), fabsf(re[i].y)));
+                m = max_nan(m, max_nan(fabsf(im[i].x), fabsf(im[i].y)));
             }
 #pragma unroll
-            for (int o = 1; o < 8; o <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+            for (int o = 1; o < 8; o <<= 1) m = max_nan(m, __shfl_xor_sync(0xffffffffu, m, o));
             // scale 2^(10 - exponent of m); at most 2^126, so that its inverse is normal
             const int bs = min(127 + 10 + 127 - (int)(__float_as_uint(m) >> 23), 253);
             const float sc = __uint_as_float((uint32_t)bs << 23);
@@ -432,16 +421,12 @@ __global__ void __launch_bounds__(XF_THREADS, 1) xengine_f32_kernel(const XfArgs
         for (int sl = 0; sl < NSLOT; sl++) {
             const long c = ch0 + sl;
             if (c >= a.nbatch) break;
-            const float2 *Xs = a.Xptrs ? a.Xptrs[c] : a.X + c * a.xstride;
             float2 *Vc = a.Vptrs ? a.Vptrs[c] : a.V + c * a.vstride;
             const float *Ds = D + sl * SLOT * XF_DS + sl * SLOT;
             auto at = [&](int r, int q) { return Ds[r * XF_DS + q]; };
             // sum over the spectra for row r, column q of the tile (r >= q on the diagonal)
             auto product = [&](int r, int q) {
-                float2 v = make_float2(at(r, q) + at(nb + r, nb + q), at(nb + r, q) - at(r, nb + q));
-                if (fail || !isfinite(v.x) || !isfinite(v.y))
-                    v = direct_product<BLOCKED>(Xs, a.ld, a.nsp, r0 + r, q0 + q);
-                return v;
+                return make_float2(at(r, q) + at(nb + r, nb + q), at(nb + r, q) - at(r, nb + q));
             };
             if (!sep) {  // the tile's square, the upper half as conjugates
                 for (int i = tid; i < nr * nr; i += 32 * XF_WARPS) {
@@ -450,12 +435,13 @@ __global__ void __launch_bounds__(XF_THREADS, 1) xengine_f32_kernel(const XfArgs
                     if (r == q) v.y = 0.f;  // autocorrelations are real
                     if (r < q) v.y = -v.y;
                     put(Vc, (long)(q0 + q) * a.ldv + r0 + r, v);
-                    if (r == q && s_uneven[sl * EB + r]) Vc[(long)(q0 + q) * a.ldv + r0 + r] = xf_mark();
+                    if (r == q && (fail || s_uneven[sl * EB + r])) Vc[(long)(q0 + q) * a.ldv + r0 + r] = xf_mark();
                 }
             } else {
                 for (int i = tid; i < nr * 64; i += 32 * XF_WARPS) {
                     const int q = i / nr, r = i - q * nr;
                     put(Vc, (long)(q0 + q) * a.ldv + r0 + r, product(r, q));
+                    if (i == 0 && fail) Vc[(long)q0 * a.ldv + r0] = xf_mark();
                 }
                 for (int i = tid; i < nr * 64; i += 32 * XF_WARPS) {
                     const int r = i >> 6, q = i & 63;
