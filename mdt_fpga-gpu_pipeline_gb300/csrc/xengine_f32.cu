@@ -50,13 +50,17 @@
 // the K-major 128-byte-swizzled operand, and adds the sums of an earlier stage from
 // tensor memory to its registers.  Two operand stages and two accumulator sets
 // alternate: while the tensor core works on stage k + 1, the warps drain stage k
-// and write stage k + 2 over its operands.  Five warpgroups share the registers: 104 for
-// a converting thread instead of 96, without which the count spills.
+// and write stage k + 2 over its operands.
 //
 // What bounds it: an M = 128, K = 16 MMA takes 63 cycles for any N up to 128, so the
-// sixteen of a stage take 1000 of the 3100 cycles that a stage takes at 40 inputs and of
-// the 4500 at 256; the rest is the warps' chain of tensor-memory reads, conversion and
-// sample loads, one after the other.
+// sixteen of a stage take 1000 of the 3150 cycles that a stage takes at 40 inputs and of
+// the 4600 at 256; the rest is the warps' chain of tensor-memory reads, conversion and
+// sample loads, one after the other.  The count takes 50 to 150 cycles of a stage, the
+// search for marks 2 us (a plan's X-engine without them: NE=10, Nch=1024, Nsp=1000 56 us,
+// with them 59; NE=32, Nsp=4096 392 and 430; NE=40, Nch=2048, Nsp=4096 1.34 and 1.39 ms;
+// NE=256, Nch=1024, Nsp=2048 4.97 and 4.93).  Against the SIMT kernel, Nch=1024, Nsp=1000:
+// NE=10 59 us, 68; NE=20 112, 104; NE=32 127, 171; NE=40 203, 229; NE=64 253, 563; NE=65
+// 683, 839; NE=128 0.78 ms, 1.85; NE=256 2.71, 6.35.
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -66,21 +70,26 @@
 
 namespace mdt {
 
-constexpr int XF_WARPS = 16;  // converting warps; then the issuing one and three without work
-// (registers are split by warpgroups).  The kernel is launched with XF_REGS registers a
-// thread; the converting warps take XF_REGS_CONV and the others keep XF_REGS_REST, the
-// same 61,440 in all.
-constexpr int XF_THREADS = 32 * (XF_WARPS + 4);
+constexpr int XF_WARPS = 16;  // converting warps, then the issuing one
+// With 128 rows a channel the issuing warp has three more without work beside it, since
+// registers are shared out by warpgroups: of the XF_REGS a thread at the launch the
+// converting ones take XF_REGS_CONV, the others keep XF_REGS_REST, the same 61,440 in all.
 constexpr int XF_REGS = 96, XF_REGS_CONV = 104, XF_REGS_REST = 64;
-static_assert(XF_REGS_CONV * 32 * XF_WARPS + XF_REGS_REST * 32 * 4 <= XF_REGS * XF_THREADS, "register split");
+constexpr int xf_threads(int slot) { return 32 * (XF_WARPS + (slot == 128 ? 4 : 1)); }
+static_assert(XF_REGS_CONV * 32 * XF_WARPS + XF_REGS_REST * 32 * 4 <= XF_REGS * xf_threads(128), "register split");
 constexpr int XF_K = 64;                          // spectra per stage
 constexpr int XF_PLANE = 128 * 128;               // 128 rows of 64 f16
 constexpr int XF_OPERAND = 2 * XF_PLANE;          // h, l
 constexpr int XF_AHEAD = 3;                       // stages between L2 prefetch and load
 constexpr int XF_FLUSH = 8;                       // stages per first-level sum
-// Spectra from which the tensor cores are used.  Shorter sums round little in
-// FP32 multiply-adds (NE=10: 6.7e-8 at 64 spectra, 8.6e-8 at 250), there the split
-// is no closer to the 64-bit sums, and there is little time to gain.
+// Spectra from which the tensor cores are used.  Shorter sums round little in FP32
+// multiply-adds (NE=10: 6.7e-8 at 64 spectra, 8.6e-8 at 250), there the split is no closer
+// to the 64-bit sums, and there is little time to gain.  At the line, Nch=1024, 256 and 400
+// spectra, here and by the SIMT kernel:  NE=3 23 and 31 us, 18 and 25;  NE=16 25 and 33, 26
+// and 37;  NE=20 41 and 55, 33 and 48;  NE=33 68 and 100, 64 and 97;  NE=64 94 and 130, 153
+// and 238;  NE=129 494 and 713, 601 and 931.  Up to 24 inputs the SIMT kernel is the faster
+// up to some 600 spectra, but rounds more (400 spectra: NE=3 5.3e-8 here, 7.1e-8; NE=20
+// 6.3e-8, 7.9e-8; NE=33 7.0e-8, 2.3e-7), so the line is the same for all.
 constexpr int XF_MIN_SPECTRA = 256;
 // A stage of an element is uneven if, of its spectra, a quarter or more have no component
 // of XF_SIG or above in the scale that brings the largest one to [1024, 2048), or if that
@@ -115,11 +124,11 @@ __device__ __forceinline__ uint32_t f16x2(float2 v)
     return r;
 }
 
-// The larger of two values; NaN if one of them is.
-__device__ __forceinline__ float max_nan(float a, float b)
+// The largest of three values; NaN if one of them is.
+__device__ __forceinline__ float max_nan(float a, float b, float c)
 {
     float r;
-    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
     return r;
 }
 
@@ -132,13 +141,17 @@ __device__ __forceinline__ void count_significant(__half2 &n, uint32_t re, uint3
     n = __hadd2(n, __hge2(__hmax2(a, b), __float2half2_rn(XF_SIG)));
 }
 
-// Of the eight lanes that hold an element, from their counts (all lanes of the warp).
+__device__ __forceinline__ int lane_significant(__half2 n)
+{
+    // 1024 + the lane's count, as f16: the low digits of its bits
+    return __half_as_ushort(__hadd(__low2half(n), __high2half(n))) & 15;
+}
+
+// Of the eight lanes that hold an element (all lanes of the warp): a byte for each element.
 __device__ __forceinline__ int total_significant(__half2 n)
 {
-    // 1024 + the lane's count, as f16: the low digits of its bits; a byte for each element
-    const uint32_t mine = __half_as_ushort(__hadd(__low2half(n), __high2half(n))) & 15;
     const int at = threadIdx.x & 24;
-    return __reduce_add_sync(0xffffffffu, mine << at) >> at & 255;
+    return __reduce_add_sync(0xffffffffu, (uint32_t)lane_significant(n) << at) >> at & 255;
 }
 
 // OFF: the grid holds tiles below the diagonal (NE > 64), with an operand of
@@ -146,7 +159,7 @@ __device__ __forceinline__ int total_significant(__half2 n)
 // BLOCKED: operand X[(k/8)*ld + e*8 + k%8] (blocks of 8 spectra, the last one
 // zero-padded), else X[k*ld + e].
 template <bool OFF, int SLOT, bool BLOCKED>
-__global__ void __launch_bounds__(XF_THREADS, 1) xengine_f32_kernel(const XfArgs a)
+__global__ void __launch_bounds__(xf_threads(SLOT), 1) xengine_f32_kernel(const XfArgs a)
 {
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -172,7 +185,13 @@ __global__ void __launch_bounds__(XF_THREADS, 1) xengine_f32_kernel(const XfArgs
     const int r0 = I * 64, q0 = J * 64;
     const int nr = min(EB, a.ne - r0), nq = min(EB, a.ne - q0);
     const int nb = OFF ? 64 : a.nb;
-    const int nstage = (a.nsp + XF_K - 1) / XF_K;
+    // Stages of 64 spectra, but the first two share what is left (32 or more each): a short
+    // one has too few for the count of significant spectra (of 16 normally distributed ones,
+    // one in 10^5 has four small ones; with a last stage of 16 of 400 spectra, some channel
+    // nearly always went to xengine_simt_redo, 152 us for 105 at NE=38, Nch=1024).
+    const int nstage = (a.nsp + XF_K - 1) / XF_K;              // four or more (XF_MIN_SPECTRA)
+    const int two = 2 * XF_K - (nstage * XF_K - a.nsp) / 8 * 8;  // of the first two together
+    const int first = (two / 2 + 7) / 8 * 8;                   // of the first
 
     if (tid == 0) {
         for (int i = 0; i < 2; i++) {
@@ -192,7 +211,7 @@ __global__ void __launch_bounds__(XF_THREADS, 1) xengine_f32_kernel(const XfArgs
     const uint32_t tmem = tmem_slot;
 
     if (warp >= XF_WARPS) {
-        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(XF_REGS_REST));
+        if constexpr (SLOT == 128) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(XF_REGS_REST));
         if (warp == XF_WARPS && lane == 0) {
             // ---------------- MMA issuer: h h' to columns 0..127 of the stage's set,
             // the products with l to columns 128..255
@@ -222,7 +241,7 @@ __global__ void __launch_bounds__(XF_THREADS, 1) xengine_f32_kernel(const XfArgs
         }
         __syncwarp();
     } else {
-        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(XF_REGS_CONV));
+        if constexpr (SLOT == 128) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(XF_REGS_CONV));
         // ---------------- converting warps.  A thread takes element e of channel
         // slot g and the spectra 8 (4 sg + i) + 2 p + {0, 1}, i < 4, of a stage: in
         // the blocked layout four lanes (p) read 64 contiguous bytes, and a warp's
@@ -235,32 +254,33 @@ __global__ void __launch_bounds__(XF_THREADS, 1) xengine_f32_kernel(const XfArgs
         const float2 *xa = Xc + (BLOCKED ? (long)(r0 + e) * 8 : (long)(r0 + e));
         const float2 *xb = Xc + (BLOCKED ? (long)(q0 + e) * 8 : (long)(q0 + e));
         float2 re[4], im[4];  // the two spectra of run i
-        auto load = [&](const float2 *x, bool live, int k) {
+        // spectra s0 .. s0 + 63, but none from s1 on
+        auto load = [&](const float2 *x, bool live, int s0, int s1) {
 #pragma unroll
             for (int i = 0; i < 4; i++) {
-                const int s = k * XF_K + 8 * (4 * sg + i);
+                const int s = s0 + 8 * (4 * sg + i);
                 if constexpr (BLOCKED) {
-                    const float4 v = live && s < a.nsp
+                    const float4 v = live && s < s1
                                          ? __ldg(reinterpret_cast<const float4 *>(x + (long)(s >> 3) * a.ld) + p)
                                          : make_float4(0.f, 0.f, 0.f, 0.f);
                     re[i] = make_float2(v.x, v.z);
                     im[i] = make_float2(v.y, v.w);
                 } else {
                     const int s2 = s + 2 * p;
-                    const float2 u = live && s2 < a.nsp ? __ldg(x + (long)s2 * a.ld) : make_float2(0.f, 0.f);
-                    const float2 v = live && s2 + 1 < a.nsp ? __ldg(x + (long)(s2 + 1) * a.ld)
-                                                            : make_float2(0.f, 0.f);
+                    const float2 u = live && s2 < s1 ? __ldg(x + (long)s2 * a.ld) : make_float2(0.f, 0.f);
+                    const float2 v = live && s2 + 1 < s1 ? __ldg(x + (long)(s2 + 1) * a.ld)
+                                                         : make_float2(0.f, 0.f);
                     re[i] = make_float2(u.x, v.x);
                     im[i] = make_float2(u.y, v.y);
                 }
             }
             // into L2, XF_AHEAD stages further on
             if constexpr (BLOCKED) {
-                const int s = (k + XF_AHEAD) * XF_K + 8 * (4 * sg + p);
+                const int s = s0 + XF_AHEAD * XF_K + 8 * (4 * sg + p);
                 if (live && s < a.nsp && !(e & 1))
                     asm volatile("prefetch.global.L2 [%0];" ::"l"(x + (long)(s >> 3) * a.ld));
             } else {
-                const int s = (k + XF_AHEAD) * XF_K + 8 * (4 * sg + p) + 2 * (e & 3);
+                const int s = s0 + XF_AHEAD * XF_K + 8 * (4 * sg + p) + 2 * (e & 3);
                 if (live && s < a.nsp) {
                     asm volatile("prefetch.global.L2 [%0];" ::"l"(x + (long)s * a.ld));
                     if (s + 1 < a.nsp)
@@ -274,11 +294,11 @@ __global__ void __launch_bounds__(XF_THREADS, 1) xengine_f32_kernel(const XfArgs
             float m = 0.0f;
 #pragma unroll
             for (int i = 0; i < 4; i++) {
-                m = max_nan(m, max_nan(fabsf(re[i].x), fabsf(re[i].y)));
-                m = max_nan(m, max_nan(fabsf(im[i].x), fabsf(im[i].y)));
+                m = max_nan(m, fabsf(re[i].x), fabsf(re[i].y));
+                m = max_nan(m, fabsf(im[i].x), fabsf(im[i].y));
             }
 #pragma unroll
-            for (int o = 1; o < 8; o <<= 1) m = max_nan(m, __shfl_xor_sync(0xffffffffu, m, o));
+            for (int o = 1; o < 8; o <<= 1) m = max_nan(m, m, __shfl_xor_sync(0xffffffffu, m, o));
             // scale 2^(10 - exponent of m); at most 2^126, so that its inverse is normal
             const int bs = min(127 + 10 + 127 - (int)(__float_as_uint(m) >> 23), 253);
             const float sc = __uint_as_float((uint32_t)bs << 23);
@@ -314,11 +334,15 @@ __global__ void __launch_bounds__(XF_THREADS, 1) xengine_f32_kernel(const XfArgs
             return m >= 1.0f / (1ll << XF_EXP) && m <= (float)(1ll << XF_EXP) ? nsig : none;
         };
         bool uneven = false;
-        auto check = [&](int k, __half2 nsig) {
-            const int n = min(XF_K, a.nsp - k * XF_K);
+        auto check = [&](int n, __half2 nsig) {  // n: spectra of the stage
             if (!sep) {
-                const int sig = total_significant(nsig);  // by all lanes
-                uneven |= sig < n - (n - 1) / 4;
+                // a quarter of 64 spectra are two or more of some lane's eight, which few warps
+                // have (asking first gains 6 us of 399 at NE=20, Nsp=4096, but costs 20 of 1376
+                // with OFF at NE=129, Nch=512, Nsp=2048)
+                if (OFF || n < XF_K || __any_sync(0xffffffffu, lane_significant(nsig) <= 6)) {
+                    const int sig = total_significant(nsig);  // by all lanes
+                    uneven |= sig < n - (n - 1) / 4;
+                }
             }
         };
         auto arrive = [&](int k) {  // operands of stage k written, sums of stage k - 2 read
@@ -375,17 +399,18 @@ __global__ void __launch_bounds__(XF_THREADS, 1) xengine_f32_kernel(const XfArgs
             }
         };
         bool ok = true;
-        for (int k = 0; k < min(2, nstage); k++) {
-            load(xa, liveA, k);
+        for (int k = 0; k < 2; k++) {
+            const int s0 = k ? first : 0, s1 = k ? two : first;
+            load(xa, liveA, s0, s1);
             const __half2 nsig = convert(k, 0, liveA);
             if (sep) {
-                load(xb, liveB, k);
+                load(xb, liveB, s0, s1);
                 convert(k, 1, liveB);
             }
             arrive(k);
-            check(k, nsig);
+            check(s1 - s0, nsig);
         }
-        if (nstage > 2) load(xa, liveA, 2);
+        load(xa, liveA, two, a.nsp);
         for (int k = 0; k < nstage; k++) {
             const int s = k & 1;
             // the products are complete; all warps' scales of the stage are written
@@ -399,14 +424,14 @@ __global__ void __launch_bounds__(XF_THREADS, 1) xengine_f32_kernel(const XfArgs
             __half2 nsig;
             if (more) {
                 nsig = convert(k + 2, 0, liveA);
-                if (sep) load(xb, liveB, k + 2);
+                if (sep) load(xb, liveB, two + k * XF_K, a.nsp);
             }
             if (k % XF_FLUSH == XF_FLUSH - 1) flush(k < XF_FLUSH);
             if (more) {
                 if (sep) convert(k + 2, 1, liveB);
                 arrive(k + 2);
-                if (k + 3 < nstage) load(xa, liveA, k + 3);
-                check(k + 2, nsig);
+                if (k + 3 < nstage) load(xa, liveA, two + (k + 1) * XF_K, a.nsp);
+                check(min(XF_K, a.nsp - two - k * XF_K), nsig);
             }
         }
         if (!ok && lane == 0) atomicExch(&s_fail, 1);
@@ -497,29 +522,29 @@ mdt_status xengine_herm_f32(int ne, long nbatch, int nsp, const float2 *X,
     a.vstride = vstride;
     a.alpha = alpha;
     a.nbatch = nbatch;
-    auto launch = [&](auto kern, bool off, long blocks) -> mdt_status {
+    auto launch = [&](auto kern, bool off, int slot, long blocks) -> mdt_status {
         if (blocks > 0x7fffffffL) return invalid("xengine: grid too large");
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)xf_smem(off));
         if (e != cudaSuccess) return cuda_status(e, "xengine smem attribute");
-        if (!split_fits(kern)) return invalid("xengine: compiled with too few registers to split");
-        kern<<<(unsigned)blocks, XF_THREADS, xf_smem(off), stream>>>(a);
+        if (slot == 128 && !split_fits(kern)) return invalid("xengine: compiled with too few registers to split");
+        kern<<<(unsigned)blocks, xf_threads(slot), xf_smem(off), stream>>>(a);
         const mdt_status st = launch_status("xengine_f32_kernel");
         if (st != MDT_SUCCESS) return st;
         return xengine_simt_redo(ne, nbatch, nsp, X, Xptrs, ld, xstride, V, Vptrs, ldv, vstride, alpha,
                                  make_float2(0.f, 0.f), true, false, stream, blocked);
     };
     if (ne > 64)
-        return blocked ? launch(xengine_f32_kernel<true, 128, true>, true, nbatch * a.npairs)
-                       : launch(xengine_f32_kernel<true, 128, false>, true, nbatch * a.npairs);
+        return blocked ? launch(xengine_f32_kernel<true, 128, true>, true, 128, nbatch * a.npairs)
+                       : launch(xengine_f32_kernel<true, 128, false>, true, 128, nbatch * a.npairs);
     if (ne > 32)
-        return blocked ? launch(xengine_f32_kernel<false, 128, true>, false, nbatch)
-                       : launch(xengine_f32_kernel<false, 128, false>, false, nbatch);
+        return blocked ? launch(xengine_f32_kernel<false, 128, true>, false, 128, nbatch)
+                       : launch(xengine_f32_kernel<false, 128, false>, false, 128, nbatch);
     if (ne > 16)
-        return blocked ? launch(xengine_f32_kernel<false, 64, true>, false, cdiv(nbatch, 2))
-                       : launch(xengine_f32_kernel<false, 64, false>, false, cdiv(nbatch, 2));
-    return blocked ? launch(xengine_f32_kernel<false, 32, true>, false, cdiv(nbatch, 4))
-                   : launch(xengine_f32_kernel<false, 32, false>, false, cdiv(nbatch, 4));
+        return blocked ? launch(xengine_f32_kernel<false, 64, true>, false, 64, cdiv(nbatch, 2))
+                       : launch(xengine_f32_kernel<false, 64, false>, false, 64, cdiv(nbatch, 2));
+    return blocked ? launch(xengine_f32_kernel<false, 32, true>, false, 32, cdiv(nbatch, 4))
+                   : launch(xengine_f32_kernel<false, 32, false>, false, 32, cdiv(nbatch, 4));
 }
 
 }  // namespace mdt
