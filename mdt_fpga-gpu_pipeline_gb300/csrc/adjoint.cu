@@ -24,7 +24,10 @@ namespace mdt {
 // 2005), which is as accurate as a sum in twice the working precision (2^-48).
 // The GPU's FP64 rate is a hundredth of its FP32 rate: sums kept in double
 // held the two gradient kernels below on the FP64 pipe.  Infinities and NaN
-// leave NaN in lo; the kernels then repeat the thread's sum in double.
+// leave NaN in lo, and the error of a product below 2^-102 is no longer an FP32
+// number (that of a sum of 2^-80 and above does not miss it).  settled() is false
+// in both cases, and the kernels repeat the thread's sums in double, unless SumAny
+// finds that every product is zero.
 struct Sum2 {
     float hi = 0.0f, lo = 0.0f;
     __device__ __forceinline__ void add(float a, float b)
@@ -37,13 +40,26 @@ struct Sum2 {
         hi = s;
         lo = __fadd_rn(lo, __fadd_rn(e, d));
     }
-    __device__ __forceinline__ bool finite() const { return isfinite(hi) && isfinite(lo); }
+    __device__ __forceinline__ bool settled() const
+    {
+        const float v = fabsf(hi + lo);
+        return v >= 0x1p-80f && v < __int_as_float(0x7f800000);
+    }
     __device__ __forceinline__ double value() const { return (double)hi + (double)lo; }
+};
+struct SumAny {
+    bool any = false;
+    __device__ __forceinline__ void add(float a, float b)
+    {
+        any = any || (a != 0.0f && b != 0.0f) || !isfinite(a) || !isfinite(b);
+    }
+    __device__ __forceinline__ bool settled() const { return !any; }
+    __device__ __forceinline__ double value() const { return 0.0; }
 };
 struct SumD {
     double v = 0.0;
     __device__ __forceinline__ void add(float a, float b) { v += (double)a * (double)b; }
-    __device__ __forceinline__ bool finite() const { return true; }
+    __device__ __forceinline__ bool settled() const { return true; }
     __device__ __forceinline__ double value() const { return v; }
 };
 
@@ -129,7 +145,7 @@ __device__ __forceinline__ bool gain_sums(int ne, int nsp, int ph, const float2 
     bool ok = true;
 #pragma unroll
     for (int v = 0; v < VEC; v++) {
-        ok = ok && ar[v].finite() && ai[v].finite();
+        ok = ok && ar[v].settled() && ai[v].settled();
         re[v] = ar[v].value();
         im[v] = ai[v].value();
     }
@@ -150,7 +166,8 @@ __global__ void __launch_bounds__(32 * GG_PH, 4)
     if (in) {
         const long c = j / ev, e = (j - c * ev) * VEC;
         const long base = c * nsp * (long)ne + e;
-        if (!gain_sums<VEC, Sum2>(ne, nsp, ph, dY + base, X + base, re, im))
+        if (!gain_sums<VEC, Sum2>(ne, nsp, ph, dY + base, X + base, re, im) &&
+            !gain_sums<VEC, SumAny>(ne, nsp, ph, dY + base, X + base, re, im))
             gain_sums<VEC, SumD>(ne, nsp, ph, dY + base, X + base, re, im);
     }
 #pragma unroll
@@ -458,7 +475,7 @@ __device__ __forceinline__ bool tap_sums(int nch, int ne, int nsp, int len, int 
     for (int i = 0; i < NT; i++)
 #pragma unroll
         for (int v = 0; v < VEC; v++) {
-            ok = ok && acc[i][v].finite();
+            ok = ok && acc[i][v].settled();
             out[i][v] = acc[i][v].value();
         }
     return ok;
@@ -474,7 +491,8 @@ __global__ void __launch_bounds__(32 * TG_PH, NT * VEC <= 8 ? 2 : 1)
     const int ph = threadIdx.y, p = blockIdx.y;
     const long first = (long)p * TG_PH + ph, stride = (long)nsplit * TG_PH;
     double sum[NT][VEC] = {};
-    if (k < nch && !tap_sums<NT, VEC, Sum2>(nch, ne, nsp, len, k, first, stride, gP, iq, sum))
+    if (k < nch && !tap_sums<NT, VEC, Sum2>(nch, ne, nsp, len, k, first, stride, gP, iq, sum) &&
+        !tap_sums<NT, VEC, SumAny>(nch, ne, nsp, len, k, first, stride, gP, iq, sum))
         tap_sums<NT, VEC, SumD>(nch, ne, nsp, len, k, first, stride, gP, iq, sum);
     const int tid = ph * 32 + threadIdx.x;
 #pragma unroll
