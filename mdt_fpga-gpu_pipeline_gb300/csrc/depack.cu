@@ -100,7 +100,7 @@ __global__ void depacketise_kernel(DepackGeom g, const unsigned char *__restrict
 }
 
 // The same for packets whose 32-sample runs fit a warp's staging buffer: one
-// warp per packet, DP_PER packets per warp.  Payload words are copied
+// warp per packet, `turns` packets per warp, four apart.  Payload words are copied
 // contiguously (WB = 16 bytes where the packets' alignment allows it, else 4)
 // into one of the warp's two buffers with cp.async, the next packet's before
 // this one's header is looked at, and written with the lanes along the samples
@@ -110,7 +110,7 @@ __global__ void depacketise_kernel(DepackGeom g, const unsigned char *__restrict
 // channels and spectra, 28 samples a packet, int32: 123 us (5.2 TB/s) against
 // 205 us with a block per packet and strided 8-byte reads; without the second
 // buffer 141 us.
-constexpr int DP_WARPS = 4, DP_PER = 8;
+constexpr int DP_WARPS = 4;
 constexpr int DP_BUF = 4096;  // bytes of a staging buffer
 
 template <int WB>
@@ -132,7 +132,7 @@ __device__ __forceinline__ void copy_words(unsigned char *dst, const unsigned ch
 
 template <int WB>
 __global__ void __launch_bounds__(32 * DP_WARPS)
-    depacketise_warp_kernel(DepackGeom g, int maxn, const unsigned char *__restrict__ pkts,
+    depacketise_warp_kernel(DepackGeom g, int maxn, int turns, const unsigned char *__restrict__ pkts,
                             int npackets, void *__restrict__ out, unsigned int *__restrict__ seen,
                             mdt_depack_stats *__restrict__ stats)
 {
@@ -146,15 +146,15 @@ __global__ void __launch_bounds__(32 * DP_WARPS)
     // the first run of a packet, sized for the widest SNAP (inside the packet
     // whatever its SNAP is: packet_bytes holds the widest payload)
     const int lead = (min(32, g.sper) * maxn * per + WB - 1) / WB;
-    const long pk0 = (long)blockIdx.x * (DP_PER * DP_WARPS) + warp;
+    const long pk0 = (long)blockIdx.x * (turns * DP_WARPS) + warp;
     const unsigned char *pay = pkts + 4 * g.hdr_words;
     if (pk0 < npackets) copy_words<WB>(sbuf[warp][0], pay + pk0 * g.pkt_bytes, lead, lane);
-    for (int m = 0; m < DP_PER; m++) {
+    for (int m = 0; m < turns; m++) {
         const long pk = pk0 + (long)m * DP_WARPS;
         if (pk >= npackets) break;
         unsigned char *buf = sbuf[warp][m & 1];
         // the packet after this one (an empty group when there is none)
-        const bool more = m + 1 < DP_PER && pk + DP_WARPS < npackets;
+        const bool more = m + 1 < turns && pk + DP_WARPS < npackets;
         copy_words<WB>(sbuf[warp][(m + 1) & 1], pay + (pk + DP_WARPS) * g.pkt_bytes,
                        more ? lead : 0, lane);
         const uint32_t *hdr = (const uint32_t *)(pkts + pk * g.pkt_bytes);
@@ -346,17 +346,21 @@ MDT_API mdt_status mdt_depacketise(const mdt_packet_format *fmt, const void *pac
     int maxn = 0;
     for (int k = 0; k < fmt->nsnap; k++) maxn = std::max(maxn, fmt->inputs_per_snap[k]);
     if ((long)maxn * 32 * (fmt->sample_bits == 32 ? 8 : 2) <= mdt::DP_BUF) {
-        const unsigned blocks = (unsigned)mdt::cdiv(npackets, mdt::DP_WARPS * mdt::DP_PER);
+        // As many packets per warp, up to eight, as fill the GPU with six blocks an SM: a
+        // warp takes its packets one after the other (588 packets of int32, eight each: 13.3
+        // us; @@SMALL@@).
+        const int turns = (int)std::max<long>(1, std::min<long>(8, npackets / (6L * mdt::DP_WARPS * mdt::sm_count())));
+        const unsigned blocks = (unsigned)mdt::cdiv(npackets, mdt::DP_WARPS * turns);
         // 16-byte reads where every payload starts on a 16-byte boundary and the
         // packet stride keeps the last read inside the packet
         const bool wide = (((uintptr_t)packets | (uintptr_t)fmt->packet_bytes |
                             (uintptr_t)(4L * fmt->words_header)) & 15) == 0;
         if (wide)
             mdt::depacketise_warp_kernel<16><<<blocks, 32 * mdt::DP_WARPS, 0, stream>>>(
-                g, maxn, (const unsigned char *)packets, npackets, out, seen, stats);
+                g, maxn, turns, (const unsigned char *)packets, npackets, out, seen, stats);
         else
             mdt::depacketise_warp_kernel<4><<<blocks, 32 * mdt::DP_WARPS, 0, stream>>>(
-                g, maxn, (const unsigned char *)packets, npackets, out, seen, stats);
+                g, maxn, turns, (const unsigned char *)packets, npackets, out, seen, stats);
         return mdt::launch_status("depacketise_warp_kernel");
     }
     mdt::depacketise_kernel<<<(unsigned)npackets, 128, 0, stream>>>(
