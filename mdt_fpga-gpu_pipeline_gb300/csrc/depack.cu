@@ -348,7 +348,7 @@ MDT_API mdt_status mdt_depacketise(const mdt_packet_format *fmt, const void *pac
     if ((long)maxn * 32 * (fmt->sample_bits == 32 ? 8 : 2) <= mdt::DP_BUF) {
         // As many packets per warp, up to eight, as fill the GPU with six blocks an SM: a
         // warp takes its packets one after the other (588 packets of int32, eight each: 13.3
-        // us; @@SMALL@@).
+        // us, one each 3.3; 9364, eight 14.1, two 10.3).
         const int turns = (int)std::max<long>(1, std::min<long>(8, npackets / (6L * mdt::DP_WARPS * mdt::sm_count())));
         const unsigned blocks = (unsigned)mdt::cdiv(npackets, mdt::DP_WARPS * turns);
         // 16-byte reads where every payload starts on a 16-byte boundary and the
