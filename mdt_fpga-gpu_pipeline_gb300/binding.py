@@ -179,7 +179,10 @@ def stream_handle(stream=None):
     if stream is None:
         import torch
         # the handle alone: current_stream() builds a Stream object, 4 us a call
-        return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+        raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)  # not a public function
+        if raw is not None:
+            return raw(torch.cuda.current_device())
+        return torch.cuda.current_stream().cuda_stream
     if isinstance(stream, int):
         return stream
     return stream.cuda_stream
