@@ -10,11 +10,14 @@
 // bits below the largest component.  A product of two samples is
 //   (x s)(y t) = h h' + (h l' + l h' + l l'),
 // exact f16 products all.  The h h' sum is kept apart from the others: it is a
-// sum of integers, exact in FP32 below 2^24 (about its size for noise-like samples;
-// beyond, it loses a unit in the last place).  That matters because the tensor
+// sum of integers, exact in FP32 below 2^24.  That matters because the tensor
 // core truncates when it adds to its accumulator: sums with fractions lose half a
 // unit per step, always towards zero (f16 pairs split by value: autocorrelations
-// 2.3e-7 low after 64 spectra).  The stage's sums go to FP32 registers, XF_FLUSH
+// 2.3e-7 low after 64 spectra).  Noise reaches 2^23 to 2^25 (autocorrelations 0.3e-7
+// low), a tone of constant amplitude 2^28: its autocorrelations come out 0.7e-7 to
+// 1.5e-7 low, with an error of 1.1e-7 (SIMT kernel: 0.6e-7 at 10 inputs, 1.6e-7 to
+// 6e-7 at 40).  Half the scale ends that (0.2e-7), but costs products of unlike
+// elements a bit (noise, 1000 spectra: 3.3e-7 for 1.8e-7; SIMT 2.2e-7).  The stage's sums go to FP32 registers, XF_FLUSH
 // stages at a time and then to a second level, so that a visibility of 1000
 // spectra is rounded about ten times, not a thousand times.
 // Relative error of V against 64-bit sums of the same FP32 samples (normal
