@@ -125,8 +125,10 @@ MDT_API mdt_status mdt_window_hamming_sinc(int nchannels, int ntaps, float *wind
 MDT_API mdt_status mdt_fft_c2c(const void *in, void *out, long rows, int n, int direction,
                                cudaStream_t stream);
 
-/* Hermitian X-engine, FP32 (from 256 spectra on as exact products of split
- * samples on the tensor cores, else SIMT):  for each channel c,
+/* Hermitian X-engine, FP32 (from 256 spectra on as products of split samples
+ * on the tensor cores, but for elements with samples of very uneven size, of
+ * extreme size or not finite, which go to a second kernel; else SIMT):  for
+ * each channel c,
  *   V_c = alpha * X_c X_c^H   (X_c = NE x Nsp column-major with leading
  *   dimension ld >= NE, base X + c*xstride complex values), written full square
  *   column-major with leading dimension NE at V + c*NE*NE.  Only the lower
@@ -276,7 +278,10 @@ MDT_API mdt_status mdt_fx_set_window(mdt_fx_plan plan, const float *window);
  * [Nch][NE*NE], 16-byte aligned, zeroed by the caller) is set, every
  * integration's visibilities are also added into it; NULL disables.  An FP32
  * plan then computes them on the SIMT cores whatever its size, so that a sum
- * kept from before continues with terms rounded the same way. */
+ * kept from before continues with the same terms.  From 256 spectra on the
+ * visibilities that it returns then differ in rounding from those without an
+ * accumulator (by some 1e-7 of their size at 10 elements to 1e-6 at 256, by
+ * which they are the less exact ones), and take up to 2.5 times as long. */
 MDT_API mdt_status mdt_fx_set_accumulator(mdt_fx_plan plan, void *acc);
 /* INT8 plans: per-channel requantisation scales (device, Nch floats).  The
  * F-output x of channel c becomes clamp(rint(x * scales[c]), -127, 127);

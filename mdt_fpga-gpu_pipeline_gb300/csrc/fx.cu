@@ -144,8 +144,8 @@ mdt_status one_integration(mdt_fx_plan p, const int8_t *hist, int nhist, const i
     if (d.precision == MDT_PREC_FP32) {
         // F-output in the 8-spectrum blocked layout XB (fengine.cuh)
         const long nsb = (d.nspectra + 7) / 8;
-        // An FP64 sum over integrations may be saved and continued later: its terms come
-        // from the one kernel that rounds the same way at every number of spectra.
+        // An FP64 sum over integrations may be saved and continued later: its terms keep the
+        // bits that they had before there was another X-engine.
         const auto xengine = p->acc ? mdt::xengine_simt_f32 : mdt::xengine_herm_f32;
         if (d.nchannels <= 2048)
             st = mdt::fengine_c64b(d.nelements, d.nchannels, d.ntaps, d.nspectra, hist, nhist, iq,

@@ -1,5 +1,7 @@
 // xengine_simt.cu -- FP32 (SIMT) X-engine, for integrations of fewer spectra
-// than the tensor-core form takes (xengine_f32.cu): per channel c the Hermitian
+// than the tensor-core form takes (xengine_f32.cu), for plans with an FP64 sum
+// over integrations, for calls with beta, and for the elements that the
+// tensor-core form leaves to it: per channel c the Hermitian
 // product V_c = alpha * X_c X_c^H (+ beta V_c), computed on the lower
 // triangle only and mirrored, which is the reference's cublasCgemmBatched
 // call (OP_N, OP_C, A == B, alpha = 1/Nspectra, beta = 0;
